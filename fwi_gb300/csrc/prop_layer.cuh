@@ -439,7 +439,7 @@ k_adj_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int j, int ntb
     for (int k = tid; k < TH * TT; k += kTmaThreads) {
         const int rr = k / TT, cc = k - rr * TT;
         const int gx = x0 + cc, gz = z0 - kRad + rr;
-        const bool in = gx < nx && gz >= 0 && gz < nz;
+        const bool in = gx >= 0 && gx < nx && gz >= 0 && gz < nz;
         MP[rr][cc] = in ? b.mp[(long)gz * b.mpitch + gsh.x0 + gx] : 0.f;
     }
     const int c4 = 4 * (tid & 7), r = tid >> 3;
