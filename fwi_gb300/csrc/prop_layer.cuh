@@ -116,7 +116,7 @@ k_fwd_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int g, int ntb
         q.sc = 1.f;
         if (img_slot >= 0 && Cd::scaled) {
             q.sc = image_scale(b.amax[(long)s * (b.nt_max + 1) + g], (float)b.inv_dh2);
-            if (x0 == b.xbase && z0 == b.zbase) b.scale[(long)s * b.nt_max + g] = q.sc;  // tile (0, 0)
+            if (first_tile(x0, z0)) b.scale[(long)s * b.nt_max + g] = q.sc;
         }
         ps[tid] = q;
     }

@@ -185,6 +185,13 @@ __device__ __forceinline__ void tile_origin(const Batch<float> &b, int list, int
     }
 }
 
+// The tile that records a shot's image scale of a step: the one of interior point (4, 4).  (The
+// grid's first tile may hold nothing but the frame: origins down to -28.)
+__device__ __forceinline__ bool first_tile(int x0, int z0)
+{
+    return x0 <= kRad && x0 + TT > kRad && z0 <= kRad && z0 + TT > kRad;
+}
+
 // Max over the warp, one atomic per warp (values are >= 0).
 __device__ __forceinline__ void warp_max_to(float v, float *dst)
 {
@@ -281,7 +288,7 @@ k_fwd_tma(Batch<float> b, const __grid_constant__ TmaMaps maps, int g, int ntb, 
         q.sc = 1.f;
         if (img_slot >= 0 && Cd::scaled) {
             q.sc = image_scale(b.amax[(long)s * (b.nt_max + 1) + g], (float)b.inv_dh2);
-            if (x0 == b.xbase && z0 == b.zbase) b.scale[(long)s * b.nt_max + g] = q.sc;  // never: a layer tile
+            if (first_tile(x0, z0)) b.scale[(long)s * b.nt_max + g] = q.sc;
         }
         ps[tid] = q;
     }
