@@ -13,6 +13,7 @@
 #include "../../include/fwi.h"
 #include "common.cuh"
 #include "prop.h"
+#include "resident_plan.h"
 #include "tma.cuh"
 
 #include <cuda_fp16.h>
@@ -24,6 +25,8 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
+#include <mutex>
 #include <vector>
 
 namespace fwi {
@@ -617,6 +620,31 @@ struct CtxBase {
     }
 };
 
+// One batch at a time on the resident path of a device, over every context of the process: the
+// CTAs of such a launch wait on one another, so no two launches may hold part of the SMs each.
+// Given back when the stream's work is done.
+std::mutex &resident_mutex(int device)
+{
+    static std::mutex mu[64];
+    return mu[device & 63];
+}
+struct ResidentTurn {
+    std::mutex *mu;
+    cudaStream_t st;
+    ResidentTurn(std::mutex *m, cudaStream_t s) : mu(m), st(s)
+    {
+        if (mu) mu->lock();
+    }
+    ~ResidentTurn()
+    {
+        if (!mu) return;
+        cudaStreamSynchronize(st);
+        mu->unlock();
+    }
+    ResidentTurn(const ResidentTurn &) = delete;
+    ResidentTurn &operator=(const ResidentTurn &) = delete;
+};
+
 #define TRY(expr)                                        \
     do {                                                 \
         cudaError_t e_ = (expr);                         \
@@ -833,6 +861,7 @@ template <typename T> struct Ctx : CtxBase {
         drop_sections();
         for (void *p : allocs) cudaFree(p);
         for (const TileListEntry &e : tile_lists) cudaFree(e.dev);
+        if (res_x) cudaFree(res_x);
         free_observed();  // (the store's scratch and the kept model are among allocs)
         if (ss.side) cudaStreamSynchronize(ss.side);
         if (rst) cudaStreamSynchronize(rst);
@@ -1156,17 +1185,184 @@ template <typename T> struct Ctx : CtxBase {
     // Whether a batch of windows nxm wide runs on the small-shot cluster path: FP32, exact
     // adjoint, every step's images kept (the path has no checkpoint or boundary variant), the
     // window fitting a cluster's shared memory, and FWI_CLUSTER not set to 0.  Cached per width.
-    mutable std::vector<std::pair<int, bool>> cluster_fit;
-    bool cluster_path(int nxm) const
+    mutable std::vector<std::pair<int, int>> cluster_fit;
+    // shots the cluster path runs at once (0: not this path)
+    int cluster_path(int nxm) const
     {
-        if (!(sizeof(T) == 4 && use_tma && cfg.mode == FWI_MODE_EXACT && cfg.store == FWI_STORE_FULL)) return false;
+        if (!(sizeof(T) == 4 && use_tma && cfg.mode == FWI_MODE_EXACT && cfg.store == FWI_STORE_FULL)) return 0;
         if (const char *e = getenv("FWI_CLUSTER"))
-            if (atoi(e) == 0) return false;
+            if (atoi(e) == 0) return 0;
         for (const auto &c : cluster_fit)
             if (c.first == nxm) return c.second;
-        const bool ok = fwi::cluster_shot_fits(nxm, nz, cfg.cpml, store_type());
-        cluster_fit.emplace_back(nxm, ok);
-        return ok;
+        const int n = fwi::cluster_shots_at_once(nxm, nz, cfg.cpml, store_type());
+        cluster_fit.emplace_back(nxm, n);
+        return n;
+    }
+
+    // The launches of a batch on the resident path (resident_plan.h): of its forward steps, of its
+    // adjoint iterations; null: that phase runs otherwise.
+    struct ResidentRun {
+        const std::vector<fwi::ResidentSet> *fwd = nullptr, *adj = nullptr;
+        bool any() const { return fwd || adj; }
+    };
+    // Plans made for the windows of recent batches (a plan is a small search on the host).
+    struct ResidentPlan {
+        std::vector<int> windows;
+        int img_bytes = 0;  // of the images an adjoint reads; 0: forward
+        std::vector<fwi::ResidentSet> sets;
+    };
+    static constexpr size_t kResidentPlans = 8;
+    std::vector<std::unique_ptr<ResidentPlan>> resident_plans;  // least recently used first
+    uint64_t *res_x = nullptr, *res_w = nullptr;  // exchanged rows and maxima (zeroed when made)
+    size_t res_words = 0;                         // words of the exchanged rows
+    unsigned res_tag = 1;                         // the next unused step tag
+
+    const std::vector<fwi::ResidentSet> *resident_sets(const std::vector<int> &windows, int img_bytes, size_t smem)
+    {
+        for (size_t k = 0; k < resident_plans.size(); k++)
+            if (resident_plans[k]->img_bytes == img_bytes && resident_plans[k]->windows == windows) {
+                std::rotate(resident_plans.begin() + k, resident_plans.begin() + k + 1, resident_plans.end());
+                const std::vector<fwi::ResidentSet> &sets = resident_plans.back()->sets;
+                return sets.empty() ? nullptr : &sets;
+            }
+        if (resident_plans.size() >= kResidentPlans) resident_plans.erase(resident_plans.begin());
+        std::unique_ptr<ResidentPlan> p(new ResidentPlan);
+        p->windows = windows;
+        p->img_bytes = img_bytes;
+        if (!fwi::resident_plan(windows, nz, cfg.cpml, smem, n_sm, img_bytes, p->sets)) p->sets.clear();
+        resident_plans.push_back(std::move(p));
+        const std::vector<fwi::ResidentSet> &sets = resident_plans.back()->sets;
+        return sets.empty() ? nullptr : &sets;
+    }
+
+    // Which phases of a batch run resident on chip (prop_resident.cuh): FP32, windows that fit, and
+    // where it measured faster (the same shots, milliseconds on the path given -> resident; not with
+    // FWI_CLUSTER=0, the per-step passes):
+    //  - Small windows (to 12000 points) with all their clusters on the device at once keep the
+    //    cluster path: 400 steps of one 72 x 56 shot 1.91 -> 2.21, one 120 x 100 shot 2.36 -> 2.42;
+    //    beyond, 160 x 160 2.78 -> 2.69, 209 x 209 3.47 -> 2.79, 8 of them 7.39 -> 3.79.
+    //  - Forward (and with checkpoints everything): windows to 256 wide; to 400 in batches of up to
+    //    2 M points.  200 steps tiles -> resident: 40 of 209 x 800 17.5 -> 15.2, 8 of 360 x 300
+    //    3.0 -> 2.5, 12 of 400 x 400 (1.9 M points) 4.5 -> 4.3, 16 (2.6 M) 8.3 -> 8.9 (300 steps); one
+    //    500 x 200 1.7 -> 2.3 (300 steps): wide windows leave a CTA few rows and long halos.
+    //  - Adjoint of stored images: windows to 400 wide; to 640 where all shots run at once.  Tiles ->
+    //    resident: 40 of 320 x 300 11.9 -> 8.1 (200 steps), one 609 x 309 3.4 -> 2.5, three (two
+    //    launches) 6.0 -> 6.4 (300 and 400 steps).
+    bool resident_path(const std::vector<DevShot> &bs, int nxm, bool want_grad, ResidentRun &run)
+    {
+        run = ResidentRun();
+        if (sizeof(T) != 4 || !use_tma) return false;
+        if (const char *e = getenv("FWI_CLUSTER"))
+            if (atoi(e) == 0) return false;
+        const bool exact = cfg.mode == FWI_MODE_EXACT, ckpt = want_grad && cfg.store == FWI_STORE_CHECKPOINT;
+        const bool full = want_grad && cfg.store == FWI_STORE_FULL;
+        if (want_grad && !full && !(ckpt && exact)) return false;
+        const int at_once = cluster_path(nxm);
+        if ((long)nxm * nz <= 12000 && at_once && (int)bs.size() <= at_once) return false;
+        long points = 0;
+        std::vector<int> w;
+        for (const DevShot &d : bs) {
+            w.push_back(d.nx);
+            points += (long)d.nx * nz;
+        }
+        const bool fwd = nxm <= 256 || (nxm <= 400 && points <= 2000000L);
+        const size_t lim = fwd || nxm <= 640 ? fwi::resident_smem_limit() : 0;
+        if (!lim) return false;
+        if (fwd) run.fwd = resident_sets(w, 0, lim);
+        if (exact && (full ? nxm <= 640 : ckpt && run.fwd)) run.adj = resident_sets(w, (int)store_elem(), lim);
+        if (run.adj && nxm > 400 && run.adj->size() > 1) run.adj = nullptr;
+        if (ckpt && !run.adj) run.fwd = nullptr;
+        if (!run.any()) return false;
+        size_t words = 0;
+        auto need = [&](const std::vector<fwi::ResidentSet> *sets) {
+            for (size_t k = 0; sets && k < sets->size(); k++)
+                words = std::max(words, (size_t)(*sets)[k].nshots * fwi::kResSlots * nz * (*sets)[k].pitch);
+        };
+        need(run.fwd);
+        need(run.adj);
+        const size_t wmax = (size_t)fwi::kResSlots * fwi::kResMaxCtas;
+        if (words > res_words) {
+            if (res_x) cudaFree(res_x);
+            res_x = nullptr;
+            res_words = 0;
+            if (cudaMalloc(&res_x, (words + wmax) * sizeof(uint64_t)) != cudaSuccess) {
+                cudaGetLastError();  // no room for it: the other paths need none
+                res_x = nullptr;
+                run = ResidentRun();
+                return false;
+            }
+            res_w = res_x + words;
+            res_words = words;
+            res_tag = 0xffffffffu;  // zeroed before its first use (resident_tags)
+        }
+        return true;
+    }
+
+    // Tags of a launch's `steps` steps, never used before in the exchange buffer: the first of them.
+    int resident_tags(int steps, unsigned &tag)
+    {
+        if (res_tag > 0xffffffffu - (unsigned)steps - 2u) {
+            TRY(cudaMemsetAsync(res_x, 0, (res_words + (size_t)fwi::kResSlots * fwi::kResMaxCtas) * sizeof(uint64_t), st));
+            res_tag = 1;
+        }
+        tag = res_tag;
+        res_tag += (unsigned)steps + 1u;
+        return FWI_OK;
+    }
+
+    // Global steps [g0, g1) of every set; checkpoint load_ck (or zero state), the first save_ck
+    // checkpoints written, images from img_first on.
+    int resident_forward(const Batch<T> &b, const std::vector<fwi::ResidentSet> &sets, int nxm, int ntb, int g0, int g1,
+                         int img_first, int period, int load_ck, int save_ck)
+    {
+        if constexpr (sizeof(T) == 4) {
+            for (const fwi::ResidentSet &set : sets) {
+                fwi::ResFwdArgs a{};
+                unsigned tag = 0;
+                int rc = resident_tags(g1 - g0, tag);
+                if (rc) return rc;
+                a.ntb = ntb;
+                a.g0 = g0;
+                a.g1 = g1;
+                a.img_first = img_first;
+                a.period = period;
+                a.load_ck = load_ck;
+                a.save_ck = save_ck;
+                a.tile_order = !cluster_path(nxm);
+                a.plain_images = cfg.mode != FWI_MODE_EXACT;
+                a.ck = ck;
+                a.ck_stride = (long)B * slot;
+                a.x = res_x;
+                a.w = res_w;
+                a.tag0 = tag - (unsigned)g0;
+                TRY(fwi::launch_resident_forward(b, set, a, st));
+                launches++;
+            }
+        }
+        return FWI_OK;
+    }
+
+    // Adjoint iterations [j0, j1) of every set, images at slot (global step - img_base).
+    int resident_adjoint(const Batch<T> &b, const std::vector<fwi::ResidentSet> &sets, int ntb, int j0, int j1,
+                         int img_base)
+    {
+        if constexpr (sizeof(T) == 4) {
+            for (const fwi::ResidentSet &set : sets) {
+                fwi::ResAdjArgs a{};
+                unsigned tag = 0;
+                int rc = resident_tags(j1 - j0, tag);
+                if (rc) return rc;
+                a.ntb = ntb;
+                a.j0 = j0;
+                a.j1 = j1;
+                a.img_base = img_base;
+                a.x = res_x;
+                a.tag0 = tag - (unsigned)j0;
+                TRY(fwi::launch_resident_adjoint(b, set, a, st));
+                launches++;
+            }
+        }
+        return FWI_OK;
     }
 
     // Device copies of the compact tile lists (Batch::tiles), one per window width, grid
@@ -1466,8 +1662,16 @@ template <typename T> struct Ctx : CtxBase {
                 }
             if (mask_in && (rc = gather(mask, mask_in, moff, mask_dst, 1, cudaMemcpyDefault))) return rc;
             const size_t lb = (size_t)nb * slot * sizeof(T);
-            for (auto &p : lvl) TRY(cudaMemsetAsync(p, 0, lb, st));
-            for (int k = 0; k < 4; k++) TRY(cudaMemsetAsync(cp[k], 0, lb, st));
+            // small shots on chip: one cluster per shot, every step in one launch (prop_cluster.cuh);
+            // shots over the whole GPU: one launch per set of shots (prop_resident.cuh)
+            ResidentRun resident;
+            const bool on_resident = resident_path(bs, nxm, want_grad, resident);
+            const bool on_cluster = !on_resident && cluster_path(nxm);
+            ResidentTurn turn(on_resident ? &resident_mutex(cfg.device) : nullptr, st);
+            if (!resident.fwd) {
+                for (auto &p : lvl) TRY(cudaMemsetAsync(p, 0, lb, st));
+                for (int k = 0; k < 4; k++) TRY(cudaMemsetAsync(cp[k], 0, lb, st));
+            }
             TRY(cudaMemsetAsync(amax, 0, (size_t)nb * (nt_max + 1) * sizeof(float), st));
             // the adjoint's view (its groups own the gradient slots) and the forward's
             const Choices ch = choice_for(bs, nxm);
@@ -1525,8 +1729,6 @@ template <typename T> struct Ctx : CtxBase {
                 const int seg = g / ck_every;
                 return seg >= first_direct ? g - seg * ck_every + (seg & 1) * ck_every : -1;
             };
-            // small shots on chip: one cluster per shot, every step in one launch (prop_cluster.cuh)
-            const bool on_cluster = cluster_path(nxm);
             NvtxRange fwd_range("fwi forward steps");
             if constexpr (sizeof(T) == 4) {
                 if (on_cluster) {
@@ -1534,7 +1736,12 @@ template <typename T> struct Ctx : CtxBase {
                     launches++;
                 }
             }
-            rc = on_cluster ? FWI_OK : run_section(section_key(0), 1u, nsamp, spts, [&]() -> int {
+            if (resident.fwd &&
+                (rc = resident_forward(bf, *resident.fwd, nxm, ntb, 0, ntb,
+                                       !want_grad ? ntb : ckpt ? first_direct * ck_every : 0,
+                                       ckpt ? ck_every : nt_max, -1, ckpt ? first_direct : 0)))
+                return rc;
+            rc = on_cluster || resident.fwd ? FWI_OK : run_section(section_key(0), 1u, nsamp, spts, [&]() -> int {
                 int cur = 0;
                 for (int g = 0; g < ntb; g++) {
                     if (ckpt && g % ck_every == 0 && g / ck_every < first_direct) {
@@ -1589,6 +1796,31 @@ template <typename T> struct Ctx : CtxBase {
                                                                             slot);
                 TRY_LAUNCH();
                 launches += 2;
+            } else if (want_grad && resident.adj) {
+                NvtxRange adj_range("fwi adjoint steps + imaging");
+                for (auto &p : gs) TRY(cudaMemsetAsync(p, 0, lb, st));
+                if (!ckpt) {
+                    if ((rc = resident_adjoint(b, *resident.adj, ntb, 0, ntb, 0))) return rc;
+                } else {
+                    // segments from the last: recompute its images from the checkpoint (but the last two
+                    // segments', which the forward kept), then the adjoint iterations that image in it
+                    Batch<T> rb = bf;
+                    rb.rec = obs;  // `rec` holds the residuals now
+                    for (int seg = last_seg; seg >= 0; seg--) {
+                        const int a = seg * ck_every, e = std::min(a + ck_every, ntb), h = seg & 1;
+                        if (seg < first_direct) {
+                            if ((rc = resident_forward(rb, *resident.fwd, nxm, ntb, a, e, a, ck_every, seg, 0))) return rc;
+                            recompute_steps += e - a;
+                        }
+                        if ((rc = resident_adjoint(b, *resident.adj, ntb, ntb - e, ntb - a, a - h * ck_every))) return rc;
+                    }
+                }
+                // one gradient slot per shot
+                k_accumulate_gradient<T><<<eg((long)nx * nz), 256, 0, st>>>(grad[0], grad[1], grad[2], gs[0], gs[1],
+                                                                            gs[2], shots, nb, 1, nx, nz, mpitch, pitch,
+                                                                            slot);
+                TRY_LAUNCH();
+                launches++;
             } else if (want_grad) {
                 NvtxRange adj_range("fwi adjoint steps + imaging");
                 rc = run_section(section_key(1), 6u, nsamp, spts, [&]() -> int {

@@ -213,13 +213,22 @@ void launch_adjoint_step(const Batch<T> &b, int nx_max, int j, int ntb, int cur,
 cudaError_t prepare_fp32_kernels();
 
 // Small shots resident on chip (prop_cluster.cuh): one thread-block cluster per
-// shot takes it through every step in one launch.  cluster_shot_fits: the
-// window nx wide on an nz-row grid fits the cluster's shared memory and
-// clusters of that size can run on the current device (FP32, exact adjoint,
-// full image storage).  The launches cover every shot of the batch view.
-bool cluster_shot_fits(int nx_max, int nz, int cpml, int store_type);
+// shot takes it through every step in one launch.  cluster_shots_at_once: how
+// many such shots the current device runs side by side (FP32, exact adjoint,
+// full image storage); 0 if the window nx wide on an nz-row grid does not fit
+// the cluster's shared memory.  The launches cover every shot of the batch view.
+int cluster_shots_at_once(int nx_max, int nz, int cpml, int store_type);
 cudaError_t launch_cluster_forward(const Batch<float> &b, int nx_max, int ntb, bool images, cudaStream_t st);
 cudaError_t launch_cluster_adjoint(const Batch<float> &b, int nx_max, int ntb, cudaStream_t st);
+
+// Shots resident on chip over the whole GPU (prop_resident.cuh, resident_plan.h): the current
+// device's shared memory for a CTA (0: not available), and one launch of a set of shots.
+struct ResidentSet;
+struct ResFwdArgs;
+struct ResAdjArgs;
+size_t resident_smem_limit();
+cudaError_t launch_resident_forward(const Batch<float> &b, const ResidentSet &set, const ResFwdArgs &a, cudaStream_t st);
+cudaError_t launch_resident_adjoint(const Batch<float> &b, const ResidentSet &set, const ResAdjArgs &a, cudaStream_t st);
 
 // Boundary storage (prop_boundary.cuh): ring length per shot, saving the
 // ring of step g, and the backward rebuild of the CPML-free region.

@@ -6,9 +6,11 @@
 //   main stream:  interior tiles (prop_tma.cuh)
 // joined before the next step.  Both tile passes read only the current time
 // level and write disjoint points.  The generic passes of prop.cuh serve FP64.
-// Small shots with full storage take the other route: one thread-block cluster
+// Small shots with full storage take another route: one thread-block cluster
 // per shot runs every step of a phase in one launch (prop_cluster.cuh;
-// launch_cluster_forward / launch_cluster_adjoint below).
+// launch_cluster_forward / launch_cluster_adjoint below); windows of middle
+// size a third: one cooperative launch holds a set of shots over the whole GPU
+// (prop_resident.cuh, prop_resident.cu).
 #include <mutex>
 
 #include "prop_boundary.cuh"
@@ -288,10 +290,10 @@ bool cached_cluster_plan(int nx, int nz, int cpml, int store_type, ClusterPlan &
 
 }  // namespace
 
-bool cluster_shot_fits(int nx_max, int nz, int cpml, int store_type)
+int cluster_shots_at_once(int nx_max, int nz, int cpml, int store_type)
 {
     ClusterPlan p;
-    if (!cached_cluster_plan(nx_max, nz, cpml, store_type, p)) return false;
+    if (!cached_cluster_plan(nx_max, nz, cpml, store_type, p)) return 0;
     // every kernel may take the device's whole opt-in shared memory: one setting serves all widths
     const size_t lim = cluster_smem_limit();
     for (cudaError_t e : {cluster_attrs(k_cluster_fwd<kStoreNative>, lim),
@@ -302,9 +304,9 @@ bool cluster_shot_fits(int nx_max, int nz, int cpml, int store_type)
                           cluster_attrs(k_cluster_adj<kStoreBf16>, lim)})
         if (e != cudaSuccess) {
             cudaGetLastError();
-            return false;
+            return 0;
         }
-    // clusters of p.ncta CTAs with this much shared memory each must fit on the device
+    // clusters of p.ncta CTAs with this much shared memory each, side by side on the device
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(p.ncta);
     cfg.blockDim = dim3(kClusterThreads);
@@ -319,9 +321,9 @@ bool cluster_shot_fits(int nx_max, int nz, int cpml, int store_type)
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, k_cluster_adj<kStoreHalf>, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return 0;
     }
-    return n > 0;
+    return n;
 }
 
 cudaError_t launch_cluster_forward(const Batch<float> &b, int nx_max, int ntb, bool images, cudaStream_t st)

@@ -1,0 +1,325 @@
+// The resident path's plan (prop_resident.cuh): which shots of a batch share the GPU, which rows
+// of each shot a CTA holds, and the shared memory each CTA needs.  Host code (with the CUDA
+// headers' qualifiers), so that the plan can be checked on the CPU.
+//
+// A launch holds one CTA per SM.  A CTA owns a band of interior rows of one shot's window, every
+// column; a shot's CTAs exchange the few edge rows their z-stencils need.  The shots of a batch
+// that do not fit on the SMs at once run in several sets, one launch after another.
+#pragma once
+
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+#include "common.cuh"
+
+namespace fwi {
+
+constexpr int kResMaxCtas = 160;  // CTAs of a launch (one per SM)
+constexpr int kResMinRows = 3;    // rows of a CTA at least: its halo then comes from three neighbours either side
+constexpr int kResSlots = 4;      // copies of the exchanged rows (step modulo kResSlots)
+constexpr int kResSide = 96;      // floats of a side array's row
+constexpr int kResMaxCpml = 32;   // the widest layer whose side columns fit one
+constexpr int kResFwdOwn = 5, kResAdjOwn = 8;    // own-row arrays
+constexpr int kResFwdSide = 3, kResAdjSide = 5;  // side arrays
+// Shared row pitches the kernels are compiled for, and at each the threads of a CTA at most (the
+// fewer, the more registers each) and the rows a thread holds at most.
+constexpr int kResPitches[] = {96, 160, 224, 320, 400, 512, 640};
+constexpr int kResFwdPitch = 400;  // the widest forward kernel's
+struct ResShape {
+    int threads, fwd_rows, adj_rows;
+};
+__host__ __device__ constexpr ResShape res_shape(int pitch)
+{
+    return pitch <= 320 ? ResShape{512, 4, 4} : ResShape{640, 6, 4};
+}
+
+// The pitch for windows nx wide (rows end at a multiple of 4), 0: none.
+inline int res_pitch(int nx, bool forward)
+{
+    for (int p : kResPitches)
+        if ((nx + 3) / 4 * 4 <= p) return forward && p > kResFwdPitch ? 0 : p;
+    return 0;
+}
+
+// CTA c of a launch: rows row0 .. row0 + nrow of the interior of shot `shot`, which is the xs-th
+// of the launch and whose CTAs are first .. first + count; lanes: the segments its rows are split in.
+struct ResidentGrid {
+    int n;
+    unsigned short shot[kResMaxCtas], xs[kResMaxCtas], first[kResMaxCtas], count[kResMaxCtas], row0[kResMaxCtas],
+        nrow[kResMaxCtas], lanes[kResMaxCtas];
+};
+
+// One launch: its grid, shared row pitch (the widest window's), threads and dynamic shared memory.
+struct ResidentSet {
+    ResidentGrid grid;
+    int pitch, threads, nshots;
+    size_t smem;
+};
+
+// Arguments of one forward launch: global steps [g0, g1) of a batch whose clock runs to ntb.
+struct ResFwdArgs {
+    int ntb, g0, g1;
+    int img_first;   // images are kept from this step on (>= g1: none), in slot
+    int period;      // g - seg period + (seg & 1) period of step g, seg = g / period (nt_max: slot g)
+    int load_ck;     // checkpoint to start from, or -1: zero state
+    int save_ck;     // checkpoints 0 .. save_ck - 1 are written (step k period)
+    int tile_order;  // CPML terms rounded as the tile passes', else as the cluster path's
+    int plain_images;  // images of the plain stencils (reference mode)
+    float *ck;       // [checkpoint][8][ck_stride]
+    long ck_stride;
+    uint64_t *x;     // exchanged rows: [xs][kResSlots][nz][shared row pitch] words
+    uint64_t *w;     // exchanged maxima: [kResSlots][kResMaxCtas] words
+    unsigned tag0;   // a word of step g carries tag0 + g
+};
+
+// One adjoint launch: iterations [j0, j1); images at slot (global step - img_base).
+struct ResAdjArgs {
+    int ntb, j0, j1, img_base;
+    uint64_t *x;
+    unsigned tag0;
+};
+
+// The side layers' CPML arrays keep only the columns near the layers: column ix at ix (left,
+// ix < wl) or wl + ix - xr0 (right); windows too narrow for two separate sides keep whole rows.
+struct ResGeom {
+    int wl, xr0;
+    __host__ __device__ int col(int ix) const { return ix < wl ? ix : wl + ix - xr0; }
+};
+
+__host__ __device__ inline ResGeom res_geom(int nx, int cpml)
+{
+    ResGeom g;
+    g.wl = (cpml + 3) / 4 * 4 + 12;      // pairs with a column < cpml + 4, their 10-wide windows
+    g.xr0 = (nx - cpml - 5) / 2 * 2 - 4;  // the same from the right
+    if (g.xr0 < g.wl) {
+        g.wl = kResSide;
+        g.xr0 = 0;
+    }
+    return g;
+}
+
+// Whether a band ending before interior row `end` holds a row whose update reads the bottom
+// layer's z memory variables (from 4 rows above the layer on).
+__host__ __device__ inline bool res_bottom(int end, int nz, int cpml) { return cpml > 4 && 4 + end > nz - cpml - 4; }
+
+// Halo rows of the z-stencil field of the band [row0, end): 4, or 8 where it recomputes z memory
+// variables of its neighbours from it (bottom bands but one that holds the whole bottom zone).
+__host__ __device__ inline int res_halo(int row0, int end, int nz, int cpml)
+{
+    return res_bottom(end, nz, cpml) && (4 + row0 > nz - cpml - 4 || end < nz - 8) ? 2 * kRad : kRad;
+}
+
+// Floats of a CTA's shared arrays at row pitch pt.  Forward: F (haloed) and P, two levels of each;
+// the three models; psi_x, zeta_x and what they add to Dxx P (side columns); bottom bands also psi_z
+// (4 rows either side), zeta_z and what they add to Dzz F.  Adjoint: u_z (haloed) and u_x, two
+// levels of each; the three models and three gradients; Y_x, Z_x, a Y_x, u_x at layer points,
+// -Dx(a Y_x); bottom bands Y_z, Z_z, -Dz(a Y_z); the 16-bit images of a step.  And the CPML tables.
+// img_bytes: bytes of an image value (0: the forward).
+__host__ __device__ inline size_t res_floats(int pt, int nrow, bool wide_halo, bool bottom, int img_bytes)
+{
+    size_t rows = (size_t)(img_bytes ? kResAdjOwn : kResFwdOwn) * nrow + 2 * (nrow + (wide_halo ? 4 : 2) * kRad);
+    if (bottom) rows += (size_t)3 * nrow + 2 * kRad;
+    size_t n = rows * pt + (size_t)((img_bytes ? kResAdjSide : kResFwdSide) * nrow + 2) * kResSide +
+               (size_t)2 * (nrow + 2 * kRad);
+    if (img_bytes == 2) n = (n + 3) / 4 * 4 + (size_t)nrow * pt;
+    return n;
+}
+
+// Column pairs of a window: nq in all, nside of them (nleft left) within reach of a side layer.  A
+// CTA's threads: whole warps for the side pairs of every row segment, then the others'.
+struct ResPairs {
+    int nq, nleft, nside;
+    __host__ __device__ int side_threads(int lanes) const { return (nside * lanes + 31) / 32 * 32; }
+    __host__ __device__ int threads(int lanes) const
+    {
+        return side_threads(lanes) + ((nq - nside) * lanes + 31) / 32 * 32;
+    }
+};
+__host__ __device__ inline ResPairs res_pairs(int nx, int cpml)
+{
+    ResPairs p;
+    p.nq = (nx - 8 + 1) / 2;
+    p.nleft = p.nside = 0;
+    if (cpml > 4) {
+        p.nleft = (cpml + 1) / 2 < p.nq ? (cpml + 1) / 2 : p.nq;  // pairs at 4 + 2 k < cpml + 4
+        int right = (nx - cpml - 8) / 2;                         // first pair with 4 + 2 k + 1 > nx - cpml - 5
+        if (right < p.nleft) right = p.nleft;
+        p.nside = p.nleft + (right < p.nq ? p.nq - right : 0);
+    }
+    return p;
+}
+
+// Row segments a CTA's threads can take.
+inline int res_lanes(int nx, int pt, int cpml)
+{
+    const ResPairs p = res_pairs(nx, cpml);
+    int n = 0;
+    while (p.nq > 0 && n < 64 && p.threads(n + 1) <= res_shape(pt).threads) n++;
+    return n;
+}
+
+// The most rows a CTA of this window can hold (threads, registers, shared memory).
+inline int res_row_cap(int nx, int pt, int cpml, bool wide_halo, bool bottom, int img_bytes, size_t smem_limit)
+{
+    const ResShape sh = res_shape(pt);
+    const int most = res_lanes(nx, pt, cpml) * (img_bytes ? sh.adj_rows : sh.fwd_rows);
+    if (!pt || cpml > kResMaxCpml) return 0;
+    int n = 0;
+    while (n < most && res_floats(pt, n + 1, wide_halo, bottom, img_bytes) * sizeof(float) <= smem_limit) n++;
+    return n;
+}
+
+// Rows of a window's n CTAs: `upper` bands over the rows above the bottom zone, then `lower`
+// bands over the zone (and `extra` rows above it).  cost: the largest band's, in rows; a row of a
+// bottom band counts more (the recomputed z memory variables and their two block barriers).
+struct ResPartition {
+    int upper = 0, lower = 0, extra = 0;
+    double cost = -1.0;  // < 0: no partition
+};
+
+inline ResPartition res_partition(int nx, int pt, int nz, int cpml, int n, int img_bytes, size_t smem_limit)
+{
+    const int nzi = nz - 8, cap_u = res_row_cap(nx, pt, cpml, false, false, img_bytes, smem_limit),
+              cap_1 = res_row_cap(nx, pt, cpml, false, true, img_bytes, smem_limit),
+              cap_l = res_row_cap(nx, pt, cpml, true, true, img_bytes, smem_limit);
+    const int zone = cpml > 4 ? std::min(nzi, cpml) : 0;
+    const double lanes = std::max(1, res_lanes(nx, pt, cpml));
+    // rows a thread takes in turn
+    auto turns = [&](int rows) { return std::ceil(rows / lanes); };
+    ResPartition best;
+    for (int extra = 0; extra <= (zone ? std::min(nzi - zone, 12) : 0); extra++)
+        for (int lower = zone ? 1 : 0; lower <= (zone ? std::min(n, (zone + extra) / kResMinRows) : 0); lower++) {
+            const int upper = n - lower, rest = nzi - zone - extra;
+            if ((rest == 0) != (upper == 0)) continue;
+            const int umax = upper ? (rest + upper - 1) / upper : 0, lmax = lower ? (zone + extra + lower - 1) / lower : 0;
+            if (upper && (rest / upper < kResMinRows || umax > cap_u)) continue;
+            if (lower && ((zone + extra) / lower < kResMinRows || lmax > (lower == 1 ? cap_1 : cap_l))) continue;
+            const double cu = turns(umax), cl = lower ? turns(lmax) * 1.5 + turns(lower == 1 ? lmax : lmax + 8) * 0.7 + 1.5 : 0.0;
+            const double c = std::max(cu, cl) + 1e-2 * (cu + cl) + 1e-3 * (umax + lmax);
+            if (best.cost < 0 || c < best.cost - 1e-9) {
+                best.upper = upper;
+                best.lower = lower;
+                best.extra = extra;
+                best.cost = c;
+            }
+        }
+    return best;
+}
+
+// Row counts of a partition, top band first.
+inline std::vector<int> res_bands(const ResPartition &p, int nz, int cpml)
+{
+    const int nzi = nz - 8, zone = (cpml > 4 ? std::min(nzi, cpml) : 0) + p.extra, rest = nzi - zone;
+    std::vector<int> r;
+    for (int k = 0; k < p.upper; k++) r.push_back(rest / p.upper + (k < rest % p.upper ? 1 : 0));
+    for (int k = 0; k < p.lower; k++) r.push_back(zone / p.lower + (k < zone % p.lower ? 1 : 0));
+    return r;
+}
+
+// The launches of a batch whose shots have windows nx[0], nx[1], ...: consecutive shots share a
+// launch while their fewest CTAs fit on n_sm SMs (windows of one width: the same number in each),
+// then the SMs left go one by one to the shot with the costliest band.  False if some window does
+// not fit at all.
+inline bool resident_plan(const std::vector<int> &nx, int nz, int cpml, size_t smem_limit, int n_sm, int img_bytes,
+                          std::vector<ResidentSet> &out)
+{
+    out.clear();
+    int wmax = 0;
+    for (int w : nx) wmax = std::max(wmax, w);
+    const int pt = res_pitch(wmax, img_bytes == 0);
+    const int nb = (int)nx.size(), nzi = nz - 8, sms = std::min(n_sm, kResMaxCtas), most = std::min(sms, nzi / kResMinRows);
+    struct Width {
+        int nx, least;
+        std::vector<ResPartition> part;  // by CTA count
+    };
+    std::vector<Width> widths;
+    auto width = [&](int w) -> Width & {
+        for (Width &x : widths)
+            if (x.nx == w) return x;
+        Width x{w, 0, std::vector<ResPartition>(std::max(1, most + 1))};
+        for (int n = 1; n <= most; n++) {
+            x.part[n] = res_partition(w, pt, nz, cpml, n, img_bytes, smem_limit);
+            if (x.part[n].cost >= 0 && !x.least) x.least = n;
+            // never a costlier split than with fewer CTAs
+            if (n > 1 && x.part[n - 1].cost >= 0 && (x.part[n].cost < 0 || x.part[n].cost > x.part[n - 1].cost))
+                x.part[n] = x.part[n - 1];
+        }
+        widths.push_back(x);
+        return widths.back();
+    };
+    bool uniform = true;
+    for (int w : nx) {
+        if (width(w).least == 0) return false;
+        uniform = uniform && w == nx[0];
+    }
+    int per = nb;
+    if (uniform) {
+        const int fit = sms / width(nx[0]).least, sets = (nb + fit - 1) / fit;
+        per = (nb + sets - 1) / sets;
+    }
+    for (int s0 = 0; s0 < nb;) {
+        int s1 = s0, used = 0;
+        std::vector<int> n;
+        while (s1 < nb && s1 - s0 < per && used + width(nx[s1]).least <= sms) {
+            n.push_back(width(nx[s1]).least);
+            used += n.back();
+            s1++;
+        }
+        for (;;) {  // the SMs left
+            int pick = -1, to = 0;
+            double worst = 0.0;
+            for (int k = 0; k < (int)n.size(); k++) {
+                const Width &w = width(nx[s0 + k]);
+                int m = n[k] + 1;  // the next count that lowers this shot's cost
+                while (m <= most && w.part[m].cost >= w.part[n[k]].cost) m++;
+                if (m > most || used + m - n[k] > sms) continue;
+                if (pick < 0 || w.part[n[k]].cost > worst) {
+                    pick = k;
+                    to = m;
+                    worst = w.part[n[k]].cost;
+                }
+            }
+            if (pick < 0) break;
+            used += to - n[pick];
+            n[pick] = to;
+        }
+        ResidentSet set{};
+        set.nshots = s1 - s0;
+        ResidentGrid &g = set.grid;
+        set.pitch = pt;
+        int c = 0;
+        for (int k = 0; k < set.nshots; k++) {
+            const int w = nx[s0 + k], first = c;
+            const std::vector<int> bands = res_bands(width(w).part[n[k]], nz, cpml);
+            int row = 0;
+            for (int r : bands) {
+                g.shot[c] = (unsigned short)(s0 + k);
+                g.xs[c] = (unsigned short)k;
+                g.first[c] = (unsigned short)first;
+                g.count[c] = (unsigned short)bands.size();
+                g.row0[c] = (unsigned short)row;
+                g.nrow[c] = (unsigned short)r;
+                row += r;
+                const size_t f = res_floats(pt, r, res_halo(row - r, row, nz, cpml) > kRad, res_bottom(row, nz, cpml), img_bytes) *
+                                 sizeof(float);
+                set.smem = std::max(set.smem, f);
+                // as many segments as it has rows, if the threads allow (as many as they allow in a bottom
+                // band: its z memory variables span more rows than its own)
+                const int lanes = res_lanes(w, pt, cpml);
+                g.lanes[c] = (unsigned short)(res_bottom(row, nz, cpml) ? std::min(lanes, r + 8) : std::min(lanes, r));
+                set.threads = std::max(set.threads, res_pairs(w, cpml).threads(g.lanes[c]));
+                c++;
+            }
+        }
+        g.n = c;
+        out.push_back(set);
+        s0 = s1;
+    }
+    return true;
+}
+
+}  // namespace fwi
