@@ -3,7 +3,7 @@
 //
 // Per step and batch: one pass over the CPML strip points (memory variables
 // whose x/z derivatives the main pass needs), then one tiled main pass over
-// every (shot, 32x32 tile).  The main pass stages the two stencil fields in
+// every (shot, tile).  The main pass stages the two stencil fields in
 // shared memory with the halo only along the axis their operator needs (P
 // and the adjoint's x-combination along x, F and the z-combination along z),
 // and does all point-wise work of the step in registers: CPML zeta terms,
@@ -20,9 +20,16 @@
 
 namespace fwi {
 
-constexpr int PTX = 32, PTZ = 32, PBY = 8;  // tile and block of the main passes
+// Tile of the main passes, a point a thread, and block of the strip passes.  What bounds them is the
+// FP64 pipe (64 cycles a warp instruction on an SM quarter), so that a small grid wants its points
+// spread over every quarter of the chip: 32 x 32 tiles of 4 points a thread left 103 of 152 SMs
+// idle on a 209 x 209 grid.  Microseconds a step (forward / adjoint, with strip passes of 256 ->
+// 64 threads): 209 x 209 28.7 / 41.0 -> 14.0 / 21.8, 609 x 309 41.1 / 52.3 -> 27.1 / 36.4, 2009 x 809
+// 168 / 200 -> 151 / 188.  Tiles of 32 x 4 are within 2 % of that, of 32 x 2 5 % faster on the
+// first and 9 % slower on the last (more halo), of 32 x 8 13 % slower on the first.
+constexpr int PTX = 16, PTZ = 8;
 constexpr int PXW = PTX + 2 * kRad, PZH = PTZ + 2 * kRad;
-constexpr int kStripBlock = 256;
+template <typename T> constexpr int kStripBlock = sizeof(T) == 8 ? 64 : 256;
 
 // CPML coefficient of column ix / row iz of a grid (src/parallelcalls.cu:23-33, 41-45),
 // looked up by distance into the layer.
@@ -112,7 +119,7 @@ __device__ __forceinline__ void block_max_to(float v, float *dst)
 // ---------------------------------------------------------------- forward
 
 template <typename T>
-__global__ void __launch_bounds__(kStripBlock) k_fwd_strip(Batch<T> b, int g, int ntb, int cur)
+__global__ void __launch_bounds__(kStripBlock<T>) k_fwd_strip(Batch<T> b, int g, int ntb, int cur)
 {
     const int s = blockIdx.y;
     const DevShot sh = b.shots[s];
@@ -141,7 +148,7 @@ __global__ void __launch_bounds__(kStripBlock) k_fwd_strip(Batch<T> b, int g, in
 // parameter, so that passes with and without images execute the same
 // arithmetic (a checkpointed segment must recompute the state bit for bit).
 template <typename T, int ST, bool EXACT>
-__global__ void __launch_bounds__(PTX * PBY)
+__global__ void __launch_bounds__(PTX * PTZ)
 k_fwd_main(Batch<T> b, int g, int ntb, int cur, int img_slot)
 {
     const bool STORE = img_slot >= 0;
@@ -180,10 +187,8 @@ k_fwd_main(Batch<T> b, int g, int ntb, int cur, int img_slot)
     if (ix < nx) {
         const T *psx = b.cp[0] + so, *psz = b.cp[1] + so;
         T *zx = b.cp[2] + so, *zz = b.cp[3] + so;
-        for (int r = threadIdx.y; r < PTZ; r += PBY) {
-            const int iz = z0 + r;
-            if (iz >= nz) break;
-            if (!interior(ix, iz, nx, nz)) continue;
+        const int r = threadIdx.y, iz = z0 + r;
+        if (iz < nz && interior(ix, iz, nx, nz)) {
             const long i = (long)iz * pitch + ix;
             const T p2 = d2x_tile<T, PXW>(sP, r, c) * b.inv_dh2;
             const T r2 = d2z_tile<T, PTX>(sF, r, c) * b.inv_dh2;
@@ -241,7 +246,7 @@ __device__ __forceinline__ void adj_sources(const Batch<T> &b, const DevShot &sh
 //   Zx' = S (g + bx Zx),  Yx' = S (-Dx[S (g + ax Zx')] + bx Yx)   (and the same in z).
 // Z is ping-ponged (neighbours read the old half), Y is updated in place.
 template <typename T>
-__global__ void __launch_bounds__(kStripBlock) k_adj_strip_exact(Batch<T> b, int j, int cur, int zsel)
+__global__ void __launch_bounds__(kStripBlock<T>) k_adj_strip_exact(Batch<T> b, int j, int cur, int zsel)
 {
     const int s = blockIdx.y;
     const DevShot sh = b.shots[s];
@@ -312,7 +317,7 @@ __global__ void __launch_bounds__(kStripBlock) k_adj_strip_exact(Batch<T> b, int
 // Reference adjoint, strip pass (src/parallelcalls.cu:179-198) on the
 // dt^2-scaled model-weighted adjoint fields.
 template <typename T>
-__global__ void __launch_bounds__(kStripBlock) k_adj_strip_ref(Batch<T> b, int j, int cur)
+__global__ void __launch_bounds__(kStripBlock<T>) k_adj_strip_ref(Batch<T> b, int j, int cur)
 {
     const int s = blockIdx.y;
     const DevShot sh = b.shots[s];
@@ -359,7 +364,7 @@ __global__ void __launch_bounds__(kStripBlock) k_adj_strip_ref(Batch<T> b, int j
 //   lP^m = 2 lP - lP_old + Dxx U + (strip terms),  lF^m = 2 lF - lF_old + Dzz V + (strip terms)
 // then the residual injection and the imaging condition.
 template <typename T, int ST, bool EXACT>
-__global__ void __launch_bounds__(PTX * PBY)
+__global__ void __launch_bounds__(PTX * PTZ)
 k_adj_main(Batch<T> b, int j, int ntb, int cur, int zsel, int img_base)
 {
     using Cd = Codec<T, ST>;
@@ -377,7 +382,7 @@ k_adj_main(Batch<T> b, int j, int ntb, int cur, int zsel, int img_base)
     __shared__ T sU[PTZ][PXW];
     __shared__ T sV[PZH][PTX];
     {
-        const int nthr = PTX * PBY;
+        const int nthr = PTX * PTZ;
         const int tid = threadIdx.y * PTX + threadIdx.x;
         for (int k = tid; k < PTZ * PXW; k += nthr) {
             int r = k / PXW, cc = k - r * PXW;
@@ -410,10 +415,8 @@ k_adj_main(Batch<T> b, int j, int ntb, int cur, int zsel, int img_base)
     if (ix >= nx) return;
     T *g0 = b.g[0] + so, *g1 = b.g[1] + so, *g2 = b.g[2] + so;
     const bool near_x = ix < cpml + kRad || ix > nx - cpml - 1 - kRad;
-    for (int r = threadIdx.y; r < PTZ; r += PBY) {
-        const int iz = z0 + r;
-        if (iz >= nz) break;
-        if (!interior(ix, iz, nx, nz)) continue;
+    const int r = threadIdx.y, iz = z0 + r;
+    if (iz < nz && interior(ix, iz, nx, nz)) {
         const long i = (long)iz * pitch + ix;
         T ex = d2x_tile<T, PXW>(sU, r, c) * b.inv_dh2;
         T ez = d2z_tile<T, PTX>(sV, r, c) * b.inv_dh2;
@@ -515,7 +518,7 @@ inline dim3 strip_grid(const Batch<T> &b, int nx_max)
 {
     const StripMap sm = StripMap::make(nx_max, b.nz, b.cpml);
     long n = sm.count();
-    long blocks = (n + kStripBlock - 1) / kStripBlock;
+    long blocks = (n + kStripBlock<T> - 1) / kStripBlock<T>;
     if (blocks < 1) blocks = 1;
     return dim3((unsigned)blocks, b.B);
 }
@@ -523,8 +526,8 @@ inline dim3 strip_grid(const Batch<T> &b, int nx_max)
 template <typename T, int ST>
 inline void fwd_dispatch(const Batch<T> &b, int nx_max, int g, int ntb, int cur, int slot, bool exact, cudaStream_t st)
 {
-    if (exact) k_fwd_main<T, ST, true><<<main_grid(b, nx_max), dim3(PTX, PBY), 0, st>>>(b, g, ntb, cur, slot);
-    else k_fwd_main<T, ST, false><<<main_grid(b, nx_max), dim3(PTX, PBY), 0, st>>>(b, g, ntb, cur, slot);
+    if (exact) k_fwd_main<T, ST, true><<<main_grid(b, nx_max), dim3(PTX, PTZ), 0, st>>>(b, g, ntb, cur, slot);
+    else k_fwd_main<T, ST, false><<<main_grid(b, nx_max), dim3(PTX, PTZ), 0, st>>>(b, g, ntb, cur, slot);
 }
 
 template <typename T>
@@ -532,7 +535,7 @@ void launch_forward_step(const Batch<T> &b, int nx_max, int g, int ntb, int cur,
                          bool exact, const StepStreams &ss)
 {
     cudaStream_t st = ss.main;
-    k_fwd_strip<T><<<strip_grid(b, nx_max), kStripBlock, 0, st>>>(b, g, ntb, cur);
+    k_fwd_strip<T><<<strip_grid(b, nx_max), kStripBlock<T>, 0, st>>>(b, g, ntb, cur);
     switch (b.store_type) {
     case kStoreHalf: fwd_dispatch<T, kStoreHalf>(b, nx_max, g, ntb, cur, img_slot, exact, st); break;
     case kStoreBf16: fwd_dispatch<T, kStoreBf16>(b, nx_max, g, ntb, cur, img_slot, exact, st); break;
@@ -545,9 +548,9 @@ inline void adj_dispatch(const Batch<T> &b, int nx_max, int j, int ntb, int cur,
                          int img_base, cudaStream_t st)
 {
     if (exact)
-        k_adj_main<T, ST, true><<<main_grid(b, nx_max), dim3(PTX, PBY), 0, st>>>(b, j, ntb, cur, zsel, img_base);
+        k_adj_main<T, ST, true><<<main_grid(b, nx_max), dim3(PTX, PTZ), 0, st>>>(b, j, ntb, cur, zsel, img_base);
     else
-        k_adj_main<T, ST, false><<<main_grid(b, nx_max), dim3(PTX, PBY), 0, st>>>(b, j, ntb, cur, zsel, img_base);
+        k_adj_main<T, ST, false><<<main_grid(b, nx_max), dim3(PTX, PTZ), 0, st>>>(b, j, ntb, cur, zsel, img_base);
 }
 
 template <typename T>
@@ -555,8 +558,8 @@ void launch_adjoint_step(const Batch<T> &b, int nx_max, int j, int ntb, int cur,
                          bool exact, int img_base, const StepStreams &ss)
 {
     cudaStream_t st = ss.main;
-    if (exact) k_adj_strip_exact<T><<<strip_grid(b, nx_max), kStripBlock, 0, st>>>(b, j, cur, zsel);
-    else k_adj_strip_ref<T><<<strip_grid(b, nx_max), kStripBlock, 0, st>>>(b, j, cur);
+    if (exact) k_adj_strip_exact<T><<<strip_grid(b, nx_max), kStripBlock<T>, 0, st>>>(b, j, cur, zsel);
+    else k_adj_strip_ref<T><<<strip_grid(b, nx_max), kStripBlock<T>, 0, st>>>(b, j, cur);
     switch (b.store_type) {
     case kStoreHalf: adj_dispatch<T, kStoreHalf>(b, nx_max, j, ntb, cur, zsel, exact, img_base, st); break;
     case kStoreBf16: adj_dispatch<T, kStoreBf16>(b, nx_max, j, ntb, cur, zsel, exact, img_base, st); break;

@@ -122,7 +122,7 @@ void forward_step(const Batch<float> &b, int nx_max, int g, int ntb, int cur, in
                 else fwd_layer<ST, false, true>(b, nx_max, g, ntb, cur, slot, s);
                 return;
             }
-            k_fwd_strip<float><<<strip_grid(b, nx_max), kStripBlock, 0, s>>>(b, g, ntb, cur);
+            k_fwd_strip<float><<<strip_grid(b, nx_max), kStripBlock<float>, 0, s>>>(b, g, ntb, cur);
             if (exact) fwd_layer<ST, true, false>(b, nx_max, g, ntb, cur, slot, s);
             else fwd_layer<ST, false, false>(b, nx_max, g, ntb, cur, slot, s);
         },
@@ -142,10 +142,10 @@ void adjoint_step(const Batch<float> &b, int nx_max, int j, int ntb, int cur, in
                 return;
             }
             if (exact) {
-                k_adj_strip_exact<float><<<strip_grid(b, nx_max), kStripBlock, 0, s>>>(b, j, cur, zsel);
+                k_adj_strip_exact<float><<<strip_grid(b, nx_max), kStripBlock<float>, 0, s>>>(b, j, cur, zsel);
                 adj_layer<ST, true, false>(b, nx_max, j, ntb, cur, zsel, base, s);
             } else {
-                k_adj_strip_ref<float><<<strip_grid(b, nx_max), kStripBlock, 0, s>>>(b, j, cur);
+                k_adj_strip_ref<float><<<strip_grid(b, nx_max), kStripBlock<float>, 0, s>>>(b, j, cur);
                 adj_layer<ST, false, false>(b, nx_max, j, ntb, cur, zsel, base, s);
             }
         },
