@@ -11,7 +11,7 @@
 // as C evaluates the expression, and the results equal the reference kernels
 // run as C on the CPU bit for bit.  The per-step sequences of the reference
 // (launchPropagation: 4 kernels; launchBackPropagation: 6 kernels) run as 2
-// and 3 kernels: one pass over the CPML strip points (the memory variables
+// kernels each: one pass over the CPML strip points (the memory variables
 // whose derivatives the next pass needs), then one tiled pass that stages
 // the x- and z-halos of the stencil fields in shared memory and does every
 // point-wise update of that step.
@@ -28,7 +28,13 @@ using fwi::in_strip;
 using fwi::interior;
 using fwi::StripMap;
 
-constexpr int TX = 32, TZ = 32, BY = 8;  // 32x32 outputs per 32x8-thread block
+// A block's outputs, one a thread.  What bounds the passes is the FP64 pipe (64 cycles a warp
+// instruction on an SM quarter): small tiles spread a small grid over all of it, and the fewest
+// FP64 operations a point count (RefDiv below).  One shot of the reference's sequence, 209 x 209, 300
+// steps each way: 59.7 ms with 32 x 32 tiles of 4 points a thread, 32.2 with 16 x 8, 29.1 without
+// the separate entryPoint pass and with strip blocks of 64 threads, 21.7 with the division below;
+// 609 x 309, 100 steps: 29.2, 20.8, 20.0, 13.7.  (FP32 to FP64 by integer operations measured no faster.)
+constexpr int TX = 16, TZ = 8;
 constexpr int XW = TX + 2 * fwi::kRad, ZH = TZ + 2 * fwi::kRad;
 
 cudaError_t g_last_error = cudaSuccess;
@@ -46,31 +52,57 @@ inline dim3 tile_grid(int nx, int nz) { return dim3((nx + TX - 1) / TX, (nz + TZ
 // pair sums of neighbours are FP32 operations; the coefficients are double
 // literals, so the products, the sum and the division by dh (dh2) are FP64; the
 // caller rounds the result to FP32.
-template <typename V> __device__ __forceinline__ double ref_first(V v, float dh)
+//
+// Division by an FP32 value d in FP64, correctly rounded, from r = 1 / d rounded to nearest: a quotient
+// q0 = s r, its exact remainder by a fused multiply-add, one correction (Markstein, IBM J. Res. Dev.
+// 34, 1990).  q0 is off by at most 1.5 units in the last place, so that before its rounding the
+// corrected quotient is off by less than 2^-51 units; s / d is never a midpoint of two FP64 values,
+// nor within 2^-25 units of one (d has 24 significant bits).  Zeros, infinities and NaN pass through
+// q0.  s, a sum of products of FP32 values, is zero or at least 2^-212, so nothing underflows for d in
+// [2^-100, 2^100]; other d divide (r = 0).
+struct RefDiv {
+    float d;
+    double r;
+    RefDiv(float d_ = 1.f) : d(d_), r(d_ >= 0x1p-100f && d_ <= 0x1p100f ? 1.0 / (double)d_ : 0.0) {}
+};
+__device__ __forceinline__ double ref_div(double s, const RefDiv &v)
 {
-    return ((4 / 5.) * (v(1) - v(-1)) - (1 / 5.) * (v(2) - v(-2)) + (4 / 105.) * (v(3) - v(-3)) -
-            (1 / 280.) * (v(4) - v(-4))) /
-           dh;
+    if (v.r == 0.0) return s / (double)v.d;
+    const double q0 = s * v.r, q = __fma_rn(__fma_rn(-q0, (double)v.d, s), v.r, q0);
+    const unsigned e = (unsigned)__double2hiint(q0) & 0x7ff00000u;
+    return e != 0 && e != 0x7ff00000u ? q : q0;
 }
 
-template <typename V> __device__ __forceinline__ double ref_second(V v, float dh2)
+template <typename V> __device__ __forceinline__ double ref_first(V v, const RefDiv &dh)
 {
-    return (-(205 / 72.) * v(0) + (8 / 5.) * (v(1) + v(-1)) - (1 / 5.) * (v(2) + v(-2)) +
-            (8 / 315.) * (v(3) + v(-3)) - (1 / 560.) * (v(4) + v(-4))) /
-           dh2;
+    return ref_div((4 / 5.) * (v(1) - v(-1)) - (1 / 5.) * (v(2) - v(-2)) + (4 / 105.) * (v(3) - v(-3)) -
+                   (1 / 280.) * (v(4) - v(-4)),
+                   dh);
+}
+
+template <typename V> __device__ __forceinline__ double ref_second(V v, const RefDiv &dh2)
+{
+    return ref_div(-(205 / 72.) * v(0) + (8 / 5.) * (v(1) + v(-1)) - (1 / 5.) * (v(2) + v(-2)) +
+                   (8 / 315.) * (v(3) + v(-3)) - (1 / 560.) * (v(4) + v(-4)),
+                   dh2);
 }
 
 // Along x (s = 1) or z (s = nx) of a global array, at flat index i.
-__device__ __forceinline__ float first_g(const float *f, long i, long s, float dh)
+__device__ __forceinline__ float first_g(const float *f, long i, long s, const RefDiv &dh)
 {
     return (float)ref_first([&](int k) { return f[i + k * s]; }, dh);
 }
+// ... of the product of two arrays.
+__device__ __forceinline__ float first_vg(const float *v, const float *f, long i, long s, const RefDiv &dh)
+{
+    return (float)ref_first([&](int k) { return v[i + k * s] * f[i + k * s]; }, dh);
+}
 // From a staged x-halo tile [rows][W] (output column c, row r) or z-halo tile [rows + 8][TX].
-template <int W> __device__ __forceinline__ float second_xt(const float (*t)[W], int r, int c, float dh2)
+template <int W> __device__ __forceinline__ float second_xt(const float (*t)[W], int r, int c, const RefDiv &dh2)
 {
     return (float)ref_second([&](int k) { return t[r][c + fwi::kRad + k]; }, dh2);
 }
-__device__ __forceinline__ float second_zt(const float (*t)[TX], int r, int c, float dh2)
+__device__ __forceinline__ float second_zt(const float (*t)[TX], int r, int c, const RefDiv &dh2)
 {
     return (float)ref_second([&](int k) { return t[r + fwi::kRad + k][c]; }, dh2);
 }
@@ -127,7 +159,7 @@ __global__ void k_cpml_z(float *a_z, float *b_z, int cpml, float vmax, int nz, f
 __global__ void k_psi_f_strip(const float *__restrict__ P, const float *__restrict__ F,
                               const float *__restrict__ a_x, const float *__restrict__ b_x,
                               const float *__restrict__ a_z, const float *__restrict__ b_z,
-                              float *psi_px, float *psi_fz, StripMap sm, float dh)
+                              float *psi_px, float *psi_fz, StripMap sm, RefDiv dh)
 {
     const int nx = sm.nx;
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < sm.count();
@@ -147,7 +179,7 @@ __global__ void k_zeta_f_strip(const float *__restrict__ p2, const float *__rest
                                const float *__restrict__ a_z, const float *__restrict__ b_z,
                                const float *__restrict__ psi_px, const float *__restrict__ psi_fz,
                                float *z_px, float *z_fz, float *aten_p, float *aten_f, StripMap sm,
-                               float dh)
+                               RefDiv dh)
 {
     const int nx = sm.nx;
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < sm.count();
@@ -167,7 +199,7 @@ __global__ void k_zeta_f_strip(const float *__restrict__ p2, const float *__rest
 }
 
 __global__ void k_second_p(const float *__restrict__ P, const float *__restrict__ F, float *p2,
-                           float *r2, float dh2, int nx, int nz)
+                           float *r2, RefDiv dh2, int nx, int nz)
 {
     __shared__ float sP[TZ][XW];
     __shared__ float sF[ZH][TX];
@@ -176,13 +208,11 @@ __global__ void k_second_p(const float *__restrict__ P, const float *__restrict_
     fwi::load_zhalo<float, TX, TZ>(sF, F, x0, z0, nx, nz, nx);
     __syncthreads();
     const int c = threadIdx.x, ix = x0 + c;
-    for (int r = threadIdx.y; r < TZ; r += BY) {
-        int iz = z0 + r;
-        if (!interior(ix, iz, nx, nz)) continue;
-        long i = (long)iz * nx + ix;
-        p2[i] = second_xt<XW>(sP, r, c, dh2);
-        r2[i] = second_zt(sF, r, c, dh2);
-    }
+    const int r = threadIdx.y, iz = z0 + r;
+    if (!interior(ix, iz, nx, nz)) return;
+    const long i = (long)iz * nx + ix;
+    p2[i] = second_xt<XW>(sP, r, c, dh2);
+    r2[i] = second_zt(sF, r, c, dh2);
 }
 
 // propagator_F: leapfrog update, P+F, source, receivers (src/parallelcalls.cu:88-117)
@@ -242,7 +272,7 @@ __global__ void k_res(float *Res, const float *__restrict__ shot1, const float *
 
 // SecondDerivate_P + ZETA_F + propagator_F of one step.  The strip pass
 // (k_psi_f_strip) has already advanced psi_px/psi_fz.
-__global__ void __launch_bounds__(TX * BY)
+__global__ void __launch_bounds__(TX * TZ)
 k_fwd_main(float *p2, float *r2, float *PF, const float *__restrict__ P_pre,
            const float *__restrict__ F_pre, float *P_past, float *F_past,
            const float *__restrict__ a_x, const float *__restrict__ b_x,
@@ -250,7 +280,7 @@ k_fwd_main(float *p2, float *r2, float *PF, const float *__restrict__ P_pre,
            const float *__restrict__ psi_px, const float *__restrict__ psi_fz, float *z_px,
            float *z_fz, float *aten_p, float *aten_f, const float *__restrict__ v_hor,
            const float *__restrict__ v_po, const float *__restrict__ v_nmo,
-           const float *__restrict__ source, float *shot, float C, float dh2, float dh, int nx, int nz,
+           const float *__restrict__ source, float *shot, float C, RefDiv dh2, RefDiv dh, int nx, int nz,
            int sx, int sz, int it, int cpml)
 {
     __shared__ float sP[TZ][XW];
@@ -260,60 +290,44 @@ k_fwd_main(float *p2, float *r2, float *PF, const float *__restrict__ P_pre,
     fwi::load_zhalo<float, TX, TZ>(sF, F_pre, x0, z0, nx, nz, nx);
     __syncthreads();
     const int c = threadIdx.x, ix = x0 + c;
-    if (ix >= nx) return;
-    for (int r = threadIdx.y; r < TZ; r += BY) {
-        const int iz = z0 + r;
-        if (iz >= nz) break;
-        const long i = (long)iz * nx + ix;
-        float p2v = 0.f, r2v = 0.f, atp = 0.f, atf = 0.f;
-        if (interior(ix, iz, nx, nz)) {
-            p2v = second_xt<XW>(sP, r, c, dh2);
-            r2v = second_zt(sF, r, c, dh2);
-            p2[i] = p2v;
-            r2[i] = r2v;
-            if (in_strip(ix, iz, nx, nz, cpml)) {
-                float tx = first_g(psi_px, i, 1, dh);
-                float tz = first_g(psi_fz, i, nx, dh);
-                float zp = b_x[ix] * z_px[i] + a_x[ix] * (p2v + tx);
-                float zf = b_z[iz] * z_fz[i] + a_z[iz] * (r2v + tz);
-                z_px[i] = zp;
-                z_fz[i] = zf;
-                atp = tx + zp;
-                atf = tz + zf;
-                aten_p[i] = atp;
-                aten_f[i] = atf;
-            } else {
-                atp = aten_p[i];  // outside the layers the reference reads what is stored (zeros)
-                atf = aten_f[i];
-            }
+    const int r = threadIdx.y, iz = z0 + r;
+    if (ix >= nx || iz >= nz) return;
+    const long i = (long)iz * nx + ix;
+    float p2v = 0.f, r2v = 0.f, atp = 0.f, atf = 0.f;
+    if (interior(ix, iz, nx, nz)) {
+        p2v = second_xt<XW>(sP, r, c, dh2);
+        r2v = second_zt(sF, r, c, dh2);
+        p2[i] = p2v;
+        r2[i] = r2v;
+        if (in_strip(ix, iz, nx, nz, cpml)) {
+            float tx = first_g(psi_px, i, 1, dh);
+            float tz = first_g(psi_fz, i, nx, dh);
+            float zp = b_x[ix] * z_px[i] + a_x[ix] * (p2v + tx);
+            float zf = b_z[iz] * z_fz[i] + a_z[iz] * (r2v + tz);
+            z_px[i] = zp;
+            z_fz[i] = zf;
+            atp = tx + zp;
+            atf = tz + zf;
+            aten_p[i] = atp;
+            aten_f[i] = atf;
+        } else {
+            atp = aten_p[i];  // outside the layers the reference reads what is stored (zeros)
+            atf = aten_f[i];
         }
-        propagate_point(i, ix, iz, p2v, r2v, atp, atf, PF, P_pre, F_pre, P_past, F_past, v_hor,
-                        v_po, v_nmo, source, shot, C, dh2, nx, nz, sx, sz, it, cpml);
     }
+    propagate_point(i, ix, iz, p2v, r2v, atp, atf, PF, P_pre, F_pre, P_past, F_past, v_hor,
+                    v_po, v_nmo, source, shot, C, dh2.d, nx, nz, sx, sz, it, cpml);
 }
 
 // ----------------------------------------------------------------- fused adjoint step
 
-__global__ void k_entry_point(const float *__restrict__ P_pre, const float *__restrict__ F_pre,
-                              float *aux1, float *aux2, float *aux3, float *aux4,
+// PSI_R on aux = v lambda (entryPoint's products, made here again: the same FP32 multiplications).
+__global__ void k_psi_r_strip(const float *__restrict__ P_pre, const float *__restrict__ F_pre,
                               const float *__restrict__ v_hor, const float *__restrict__ v_po,
-                              const float *__restrict__ v_nmo, long n)
-{
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        float lp = P_pre[i], lf = F_pre[i], vp = v_po[i];
-        aux1[i] = v_hor[i] * lp;
-        aux2[i] = vp * lp;
-        aux3[i] = v_nmo[i] * lf;
-        aux4[i] = vp * lf;
-    }
-}
-
-__global__ void k_psi_r_strip(const float *__restrict__ aux1, const float *__restrict__ aux2,
-                              const float *__restrict__ aux3, const float *__restrict__ aux4,
-                              const float *__restrict__ a_x, const float *__restrict__ b_x,
+                              const float *__restrict__ v_nmo, const float *__restrict__ a_x, const float *__restrict__ b_x,
                               const float *__restrict__ a_z, const float *__restrict__ b_z,
                               float *psixcx, float *psixcz, float *psizdx, float *psizcz,
-                              StripMap sm, float dh)
+                              StripMap sm, RefDiv dh)
 {
     const int nx = sm.nx;
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < sm.count();
@@ -321,10 +335,10 @@ __global__ void k_psi_r_strip(const float *__restrict__ aux1, const float *__res
         int ix, iz;
         sm.point(k, ix, iz);
         long i = (long)iz * nx + ix;
-        float p1cx = first_g(aux1, i, 1, dh);
-        float p1cz = first_g(aux2, i, nx, dh);
-        float r1dx = first_g(aux3, i, 1, dh);
-        float r1cz = first_g(aux4, i, nx, dh);
+        float p1cx = first_vg(v_hor, P_pre, i, 1, dh);
+        float p1cz = first_vg(v_po, P_pre, i, nx, dh);
+        float r1dx = first_vg(v_nmo, F_pre, i, 1, dh);
+        float r1cz = first_vg(v_po, F_pre, i, nx, dh);
         psixcx[i] = b_x[ix] * psixcx[i] + a_x[ix] * p1cx;
         psixcz[i] = b_z[iz] * psixcz[i] + a_z[iz] * p1cz;
         psizdx[i] = b_x[ix] * psizdx[i] + a_x[ix] * r1dx;
@@ -333,7 +347,8 @@ __global__ void k_psi_r_strip(const float *__restrict__ aux1, const float *__res
 }
 
 struct AdjArgs {
-    const float *aux1, *aux2, *aux3, *aux4;
+    float *aux1, *aux2, *aux3, *aux4;
+    const float *v_hor, *v_po, *v_nmo;
     float *p2cx, *p2cz, *r2dx, *r2cz;
     const float *a_x, *b_x, *a_z, *b_z;
     const float *psixcx, *psixcz, *psizdx, *psizcz;
@@ -344,12 +359,29 @@ struct AdjArgs {
     const float *Res;
     const float *P_snap, *F_snap;
     float *gcx, *gcz, *gdx;
-    float C, dh2, dt, dh;
+    RefDiv dh2, dh;
+    float C, dt;
     int nx, nz, nt, sz, it, cpml;
 };
 
-// secondDerivate + ZETA_R + retroPropagation + GRADIENT of one adjoint step.
-__global__ void __launch_bounds__(TX * BY) k_adj_main(AdjArgs a)
+// Value v(i) at every point i of the x-halo (z-halo) tile at (x0, z0), zero off the grid.
+template <typename V> __device__ __forceinline__ void stage_x(float (*s)[XW], int x0, int z0, int nx, int nz, V v)
+{
+    for (int k = threadIdx.y * TX + threadIdx.x; k < TZ * XW; k += TX * TZ) {
+        const int r = k / XW, c = k - r * XW, gx = x0 - fwi::kRad + c, gz = z0 + r;
+        s[r][c] = gx >= 0 && gx < nx && gz < nz ? v((long)gz * nx + gx) : 0.f;
+    }
+}
+template <typename V> __device__ __forceinline__ void stage_z(float (*s)[TX], int x0, int z0, int nx, int nz, V v)
+{
+    for (int k = threadIdx.y * TX + threadIdx.x; k < ZH * TX; k += TX * TZ) {
+        const int r = k / TX, c = k - r * TX, gx = x0 + c, gz = z0 - fwi::kRad + r;
+        s[r][c] = gx < nx && gz >= 0 && gz < nz ? v((long)gz * nx + gx) : 0.f;
+    }
+}
+
+// entryPoint + secondDerivate + ZETA_R + retroPropagation + GRADIENT of one adjoint step.
+__global__ void __launch_bounds__(TX * TZ) k_adj_main(AdjArgs a)
 {
     __shared__ float s1[TZ][XW];  // aux1 = v_hor lambdaP (x-halo)
     __shared__ float s3[TZ][XW];  // aux3 = v_nmo lambdaF (x-halo)
@@ -359,75 +391,76 @@ __global__ void __launch_bounds__(TX * BY) k_adj_main(AdjArgs a)
     __shared__ float sT[ZH][TX];  // snapshot F (z-halo)
     const int nx = a.nx, nz = a.nz;
     const int x0 = blockIdx.x * TX, z0 = blockIdx.y * TZ;
-    fwi::load_xhalo<float, TX, TZ>(s1, a.aux1, x0, z0, nx, nz, nx);
-    fwi::load_xhalo<float, TX, TZ>(s3, a.aux3, x0, z0, nx, nz, nx);
+    stage_x(s1, x0, z0, nx, nz, [&](long i) { return a.v_hor[i] * a.P_pre[i]; });
+    stage_x(s3, x0, z0, nx, nz, [&](long i) { return a.v_nmo[i] * a.F_pre[i]; });
     fwi::load_xhalo<float, TX, TZ>(sS, a.P_snap, x0, z0, nx, nz, nx);
-    fwi::load_zhalo<float, TX, TZ>(s2, a.aux2, x0, z0, nx, nz, nx);
-    fwi::load_zhalo<float, TX, TZ>(s4, a.aux4, x0, z0, nx, nz, nx);
+    stage_z(s2, x0, z0, nx, nz, [&](long i) { return a.v_po[i] * a.P_pre[i]; });
+    stage_z(s4, x0, z0, nx, nz, [&](long i) { return a.v_po[i] * a.F_pre[i]; });
     fwi::load_zhalo<float, TX, TZ>(sT, a.F_snap, x0, z0, nx, nz, nx);
     __syncthreads();
     const int c = threadIdx.x, ix = x0 + c;
-    if (ix >= nx) return;
+    const int r = threadIdx.y, iz = z0 + r;
+    if (ix >= nx || iz >= nz) return;
     const float *res_row = a.Res + (long)nx * (a.nt - a.it - 1);
-    for (int r = threadIdx.y; r < TZ; r += BY) {
-        const int iz = z0 + r;
-        if (iz >= nz) break;
-        const long i = (long)iz * nx + ix;
-        const bool upd = interior(ix, iz, nx, nz);
-        float pn = 0.f, fn = 0.f;
-        if (upd) {
-            float p2cx = second_xt<XW>(s1, r, c, a.dh2);
-            float r2dx = second_xt<XW>(s3, r, c, a.dh2);
-            float p2cz = second_zt(s2, r, c, a.dh2);
-            float r2cz = second_zt(s4, r, c, a.dh2);
-            a.p2cx[i] = p2cx;
-            a.r2dx[i] = r2dx;
-            a.p2cz[i] = p2cz;
-            a.r2cz[i] = r2cz;
-            float axcx, axcz, azdx, azcz;
-            if (in_strip(ix, iz, nx, nz, a.cpml)) {
-                float dxcx = first_g(a.psixcx, i, 1, a.dh);
-                float dxcz = first_g(a.psixcz, i, nx, a.dh);
-                float dzdx = first_g(a.psizdx, i, 1, a.dh);
-                float dzcz = first_g(a.psizcz, i, nx, a.dh);
-                float bx = a.b_x[ix], ax = a.a_x[ix], bz = a.b_z[iz], az = a.a_z[iz];
-                float zxcx = bx * a.zitaxcx[i] + ax * (dxcx + p2cx);
-                float zxcz = bz * a.zitaxcz[i] + az * (dxcz + p2cz);
-                float zzdx = bx * a.zitazdx[i] + ax * (dzdx + r2dx);
-                float zzcz = bz * a.zitazcz[i] + az * (dzcz + r2cz);
-                a.zitaxcx[i] = zxcx;
-                a.zitaxcz[i] = zxcz;
-                a.zitazdx[i] = zzdx;
-                a.zitazcz[i] = zzcz;
-                axcx = zxcx + dxcx;
-                axcz = zxcz + dxcz;
-                azdx = zzdx + dzdx;
-                azcz = zzcz + dzcz;
-                a.atenxcx[i] = axcx;
-                a.atenxcz[i] = axcz;
-                a.atenzdx[i] = azdx;
-                a.atenzcz[i] = azcz;
-            } else {
-                axcx = a.atenxcx[i];
-                axcz = a.atenxcz[i];
-                azdx = a.atenzdx[i];
-                azcz = a.atenzcz[i];
-            }
-            const float k = a.dh2 * a.C;
-            pn = 2.0f * a.P_pre[i] - a.P_past[i] + k * (p2cx + axcx + r2dx + azdx);
-            fn = 2.0f * a.F_pre[i] - a.F_past[i] + k * (p2cz + r2cz + axcz + azcz);
+    const long i = (long)iz * nx + ix;
+    a.aux1[i] = s1[r][c + fwi::kRad];
+    a.aux2[i] = s2[r + fwi::kRad][c];
+    a.aux3[i] = s3[r][c + fwi::kRad];
+    a.aux4[i] = s4[r + fwi::kRad][c];
+    const bool upd = interior(ix, iz, nx, nz);
+    float pn = 0.f, fn = 0.f;
+    if (upd) {
+        float p2cx = second_xt<XW>(s1, r, c, a.dh2);
+        float r2dx = second_xt<XW>(s3, r, c, a.dh2);
+        float p2cz = second_zt(s2, r, c, a.dh2);
+        float r2cz = second_zt(s4, r, c, a.dh2);
+        a.p2cx[i] = p2cx;
+        a.r2dx[i] = r2dx;
+        a.p2cz[i] = p2cz;
+        a.r2cz[i] = r2cz;
+        float axcx, axcz, azdx, azcz;
+        if (in_strip(ix, iz, nx, nz, a.cpml)) {
+            float dxcx = first_g(a.psixcx, i, 1, a.dh);
+            float dxcz = first_g(a.psixcz, i, nx, a.dh);
+            float dzdx = first_g(a.psizdx, i, 1, a.dh);
+            float dzcz = first_g(a.psizcz, i, nx, a.dh);
+            float bx = a.b_x[ix], ax = a.a_x[ix], bz = a.b_z[iz], az = a.a_z[iz];
+            float zxcx = bx * a.zitaxcx[i] + ax * (dxcx + p2cx);
+            float zxcz = bz * a.zitaxcz[i] + az * (dxcz + p2cz);
+            float zzdx = bx * a.zitazdx[i] + ax * (dzdx + r2dx);
+            float zzcz = bz * a.zitazcz[i] + az * (dzcz + r2cz);
+            a.zitaxcx[i] = zxcx;
+            a.zitaxcz[i] = zxcz;
+            a.zitazdx[i] = zzdx;
+            a.zitazcz[i] = zzcz;
+            axcx = zxcx + dxcx;
+            axcz = zxcz + dxcz;
+            azdx = zzdx + dzdx;
+            azcz = zzcz + dzcz;
+            a.atenxcx[i] = axcx;
+            a.atenxcz[i] = axcz;
+            a.atenzdx[i] = azdx;
+            a.atenzcz[i] = azcz;
+        } else {
+            axcx = a.atenxcx[i];
+            axcz = a.atenxcz[i];
+            azdx = a.atenzdx[i];
+            azcz = a.atenzcz[i];
         }
-        const bool inj = (ix > a.cpml - 1 && ix < nx - a.cpml && iz == a.sz - 1);
-        if (!upd && inj) { pn = a.P_past[i]; fn = a.F_past[i]; }
-        if (inj) { float d = res_row[ix]; pn += d; fn += d; }
-        if (upd || inj) { a.P_past[i] = pn; a.F_past[i] = fn; }
-        if (upd) {
-            float p2 = second_xt<XW>(sS, r, c, a.dh2);
-            float r2 = second_zt(sT, r, c, a.dh2);
-            a.gcx[i] += a.dt * p2 * pn;
-            a.gcz[i] += a.dt * r2 * (pn + fn);
-            a.gdx[i] += a.dt * p2 * fn;
-        }
+        const float k = a.dh2.d * a.C;
+        pn = 2.0f * a.P_pre[i] - a.P_past[i] + k * (p2cx + axcx + r2dx + azdx);
+        fn = 2.0f * a.F_pre[i] - a.F_past[i] + k * (p2cz + r2cz + axcz + azcz);
+    }
+    const bool inj = (ix > a.cpml - 1 && ix < nx - a.cpml && iz == a.sz - 1);
+    if (!upd && inj) { pn = a.P_past[i]; fn = a.F_past[i]; }
+    if (inj) { float d = res_row[ix]; pn += d; fn += d; }
+    if (upd || inj) { a.P_past[i] = pn; a.F_past[i] = fn; }
+    if (upd) {
+        float p2 = second_xt<XW>(sS, r, c, a.dh2);
+        float r2 = second_zt(sT, r, c, a.dh2);
+        a.gcx[i] += a.dt * p2 * pn;
+        a.gcz[i] += a.dt * r2 * (pn + fn);
+        a.gdx[i] += a.dt * p2 * fn;
     }
 }
 
@@ -538,10 +571,10 @@ __global__ void k_update_lbfgs(const float *r1, const float *r2, const float *r3
     }
 }
 
-constexpr int kEltBlock = 256;
-// Grid of a grid-stride kernel: one block per kEltBlock elements, at most 16
+constexpr int kEltBlock = 256, kStripBlock = 64;
+// Grid of a grid-stride kernel: one block per `block` elements, at most 16
 // blocks per SM of the current device (the runtime caches the attribute).
-inline unsigned elt_grid(long n)
+inline unsigned elt_grid(long n, int block = kEltBlock)
 {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -550,9 +583,10 @@ inline unsigned elt_grid(long n)
         sms = 1;
     }
     const long cap = 16L * sms;
-    long b = (n + kEltBlock - 1) / kEltBlock;
+    long b = (n + block - 1) / block;
     return (unsigned)(b < cap ? (b > 0 ? b : 1) : cap);
 }
+inline unsigned strip_grid(const StripMap &sm) { return elt_grid(sm.count(), kStripBlock); }
 
 }  // namespace
 
@@ -592,7 +626,7 @@ void PSI_F_h(float *P, float *F, float *a_x, float *b_x, float *a_z, float *b_z,
 {
     StripMap sm = StripMap::make(nx, nz, CPML);
     if (sm.count() == 0) return;
-    k_psi_f_strip<<<elt_grid(sm.count()), kEltBlock>>>(P, F, a_x, b_x, a_z, b_z, psi_px, psi_fz,
+    k_psi_f_strip<<<strip_grid(sm), kStripBlock>>>(P, F, a_x, b_x, a_z, b_z, psi_px, psi_fz,
                                                          sm, dh);
     note_launch();
 }
@@ -604,7 +638,7 @@ void ZETA_F_h(float *p2, float *r2, float *P, float *F, float *a_x, float *b_x, 
     (void)P; (void)F; (void)dh2;  // unused by the reference kernel as well
     StripMap sm = StripMap::make(nx, nz, CPML);
     if (sm.count() == 0) return;
-    k_zeta_f_strip<<<elt_grid(sm.count()), kEltBlock>>>(p2, r2, a_x, b_x, a_z, b_z, psi_px,
+    k_zeta_f_strip<<<strip_grid(sm), kStripBlock>>>(p2, r2, a_x, b_x, a_z, b_z, psi_px,
                                                           psi_fz, z_px, z_fz, aten_p, aten_f, sm,
                                                           dh);
     note_launch();
@@ -631,7 +665,7 @@ void res_h(float *Res, float *shot1, float *shot2, int nx, int nz)
 void SecondDerivate_P_h(float *P_pre, float *F_pre, float *p2, float *r2, float dh2, int nx,
                         int nz)
 {
-    k_second_p<<<tile_grid(nx, nz), dim3(TX, BY)>>>(P_pre, F_pre, p2, r2, dh2, nx, nz);
+    k_second_p<<<tile_grid(nx, nz), dim3(TX, TZ)>>>(P_pre, F_pre, p2, r2, dh2, nx, nz);
     note_launch();
 }
 
@@ -647,10 +681,10 @@ void launchPropagation(cudaStream_t stream1, cudaStream_t stream2, float *PF_h, 
                          cudaMemcpyDeviceToHost, stream1));
     StripMap sm = StripMap::make(nx, nz, CPML);
     if (sm.count() > 0)
-        k_psi_f_strip<<<elt_grid(sm.count()), kEltBlock, 0, stream2>>>(
+        k_psi_f_strip<<<strip_grid(sm), kStripBlock, 0, stream2>>>(
             P_pre, F_pre, a_x, b_x, a_z, b_z, psi_px, psi_fz, sm, dh);
     // legacy default stream: waits for the copy on stream1 and the strip pass on stream2
-    k_fwd_main<<<tile_grid(nx, nz), dim3(TX, BY), 0, cudaStreamLegacy>>>(
+    k_fwd_main<<<tile_grid(nx, nz), dim3(TX, TZ), 0, cudaStreamLegacy>>>(
         p2, r2, PF, P_pre, F_pre, P_past, F_past, a_x, b_x, a_z, b_z, psi_px, psi_fz, z_px, z_fz,
         aten_p, aten_f, v_hor, v_po, v_nmo, source, shot2, C, dh2, dh, nx, nz, sx, sz, it, CPML);
     note_launch();
@@ -672,14 +706,12 @@ void launchBackPropagation(cudaStream_t stream1, cudaStream_t stream2, int nx, i
     // snapshot back to the device (src/serialcalls.cu:76); F_pre2 = P_pre2 + nx*nz
     note(cudaMemcpyAsync(P_pre2, PF_h, 2 * (size_t)nx * nz * sizeof(float),
                          cudaMemcpyHostToDevice, stream1));
-    long n = (long)nx * nz;
-    k_entry_point<<<elt_grid(n), kEltBlock, 0, stream2>>>(P_pre, F_pre, aux1, aux2, aux3, aux4,
-                                                           v_hor, v_po, v_nmo, n);
     StripMap sm = StripMap::make(nx, nz, CPML);
     if (sm.count() > 0)
-        k_psi_r_strip<<<elt_grid(sm.count()), kEltBlock, 0, stream2>>>(
-            aux1, aux2, aux3, aux4, a_x, b_x, a_z, b_z, psixcx, psixcz, psizdx, psizcz, sm, dh);
+        k_psi_r_strip<<<strip_grid(sm), kStripBlock, 0, stream2>>>(
+            P_pre, F_pre, v_hor, v_po, v_nmo, a_x, b_x, a_z, b_z, psixcx, psixcz, psizdx, psizcz, sm, dh);
     AdjArgs a;
+    a.v_hor = v_hor; a.v_po = v_po; a.v_nmo = v_nmo;
     a.aux1 = aux1; a.aux2 = aux2; a.aux3 = aux3; a.aux4 = aux4;
     a.p2cx = p2cx; a.p2cz = p2cz; a.r2dx = r2dx; a.r2cz = r2cz;
     a.a_x = a_x; a.b_x = b_x; a.a_z = a_z; a.b_z = b_z;
@@ -692,7 +724,7 @@ void launchBackPropagation(cudaStream_t stream1, cudaStream_t stream2, int nx, i
     a.C = C; a.dh2 = dh2; a.dt = dt; a.dh = dh;
     a.nx = nx; a.nz = nz; a.nt = nt; a.sz = sz; a.it = it; a.cpml = CPML;
     // legacy default stream: after the H2D copy (stream1) and the strip pass (stream2)
-    k_adj_main<<<tile_grid(nx, nz), dim3(TX, BY), 0, cudaStreamLegacy>>>(a);
+    k_adj_main<<<tile_grid(nx, nz), dim3(TX, TZ), 0, cudaStreamLegacy>>>(a);
     note_launch();
 }
 
