@@ -259,36 +259,45 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// Reduces up to 4 x 3 per-thread values into partial[block], then the last
-// block to arrive sums all partials in block order into out[4][3].
-__device__ void reduce_last_block(double (&v)[4][3], int nv, DotScratch ds, double *out)
+// Reduces NV x 3 per-thread values into partial[block]; the last block to arrive sums all partials
+// (each thread its blocks', then a fixed tree: one thread in block order took 22 us for 304 blocks)
+// into out[NV][3] and calls after(p) in thread p of 3.  Every block has read its inputs by then.
+template <int NV, typename After> __device__ void reduce_last_block(double (&v)[NV][3], DotScratch ds, double *out, After after)
 {
-    __shared__ double sm[8][12];
+    __shared__ double sm[kRedThreads / 32][NV * 3];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int a = 0; a < nv; a++)
-        for (int p = 0; p < 3; p++) {
-            double t = warp_sum(v[a][p]);
-            if (lane == 0) sm[warp][a * 3 + p] = t;
-        }
-    __syncthreads();
-    if (threadIdx.x < nv * 3) {
+    // the block's sum of each value, in threads 0 .. 3 NV - 1
+    auto block_sum = [&]() {
+        for (int a = 0; a < NV; a++)
+            for (int p = 0; p < 3; p++) {
+                const double t = warp_sum(v[a][p]);
+                if (lane == 0) sm[warp][a * 3 + p] = t;
+            }
+        __syncthreads();
         double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sm[w][threadIdx.x];
-        ds.partial[(long)blockIdx.x * 12 + threadIdx.x] = t;
-    }
+        if (threadIdx.x < NV * 3)
+            for (int w = 0; w < kRedThreads / 32; w++) t += sm[w][threadIdx.x];
+        return t;
+    };
+    const double mine = block_sum();
+    if (threadIdx.x < NV * 3) ds.partial[(long)blockIdx.x * 12 + threadIdx.x] = mine;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = (atomicAdd(ds.counter, 1u) == gridDim.x - 1);
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (threadIdx.x < nv * 3) {
-        double t = 0.0;
-        for (int bI = 0; bI < (int)gridDim.x; bI++) t += ((volatile double *)ds.partial)[(long)bI * 12 + threadIdx.x];
-        out[threadIdx.x] = t;
-    }
+    for (int a = 0; a < NV; a++)
+        for (int p = 0; p < 3; p++) {
+            v[a][p] = 0.0;
+            for (unsigned k = threadIdx.x; k < gridDim.x; k += kRedThreads) v[a][p] += __ldcg(&ds.partial[(long)k * 12 + a * 3 + p]);
+        }
+    const double sum = block_sum();
+    if (threadIdx.x < NV * 3) out[threadIdx.x] = sum;
     if (threadIdx.x == 0) *ds.counter = 0u;
+    __syncthreads();
+    if (threadIdx.x < 3) after((int)threadIdx.x);
 }
 
 template <typename T> struct Tri {
@@ -298,64 +307,27 @@ template <typename T> struct CTri {
     const T *p[3];
 };
 
-// s_k = m - m_back, y_k = g - g_back (3 parameters), and the dots y.s, y.y, s.g, s.s.
-template <typename T>
-__global__ void k_lb_pair(Tri<T> s, Tri<T> y, CTri<T> m, CTri<T> mb, CTri<T> g, CTri<T> gb, long n,
-                          DotScratch ds, double *out)
-{
-    double v[4][3] = {};
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        for (int p = 0; p < 3; p++) {
-            T sv = m.p[p][i] - mb.p[p][i], yv = g.p[p][i] - gb.p[p][i];
-            s.p[p][i] = sv;
-            y.p[p][i] = yv;
-            v[0][p] += (double)yv * sv;
-            v[1][p] += (double)yv * yv;
-            v[2][p] += (double)sv * g.p[p][i];
-            v[3][p] += (double)sv * sv;
-        }
-    reduce_last_block(v, 4, ds, out);
-}
+// 16 bytes of an array (rows are padded to 128 bytes).
+template <typename T> struct alignas(16) Pack {
+    static constexpr int N = 16 / sizeof(T);
+    T v[N];
+    __device__ __forceinline__ static Pack get(const T *p) { return *reinterpret_cast<const Pack *>(p); }
+    __device__ __forceinline__ void put(T *p) const { *reinterpret_cast<Pack *>(p) = *this; }
+};
 
-// v := w (copy) and the dots a.w for the first loop's first slot.
-template <typename T>
-__global__ void k_lb_copy_dot(Tri<T> dst, CTri<T> src, CTri<T> a, long n, DotScratch ds, double *out)
-{
-    double v[4][3] = {};
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        for (int p = 0; p < 3; p++) {
-            T w = src.p[p][i];
-            dst.p[p][i] = w;
-            v[0][p] += (double)a.p[p][i] * w;
-        }
-    reduce_last_block(v, 1, ds, out);
-}
+// The passes of the L-BFGS recursion below are bound by the FP64 pipe (64 cycles a warp instruction
+// on an SM quarter; the sums and coefficients are FP64) and, per pass, by the launch and the last
+// block's tail.  So: no FP64 multiplication that an operand of 1 or 0 makes idle, copies made by the
+// pass that has the values in registers, scalar bookkeeping in the last block of the reduction that
+// feeds it.  On a 2009 x 809 model, first step and 5 directions and updates: 4.9 -> 1.5 ms.
 
-// x := c0 * x + c1 * u (per-parameter scalars from device memory, FP64), then
-// the dots b.x for the next step (b may be null).
-template <typename T>
-__global__ void k_lb_axpy_dot(Tri<T> x, CTri<T> u, const double *c0, const double *c1, CTri<T> bnext,
-                              int has_next, long n, DotScratch ds, double *out)
-{
-    double v[4][3] = {};
-    double k0[3], k1[3];
-    for (int p = 0; p < 3; p++) { k0[p] = c0 ? c0[p] : 1.0; k1[p] = c1 ? c1[p] : 0.0; }
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        for (int p = 0; p < 3; p++) {
-            T xv = (T)(k0[p] * (double)x.p[p][i] + (u.p[p] ? k1[p] * (double)u.p[p][i] : 0.0));
-            x.p[p][i] = xv;
-            if (has_next) v[0][p] += (double)bnext.p[p][i] * xv;
-        }
-    if (has_next) reduce_last_block(v, 1, ds, out);
-}
-
-// Scalar bookkeeping of the two-loop recursion (one thread).
+// Scalars of the two-loop recursion.
 struct LbScalars {
     double rho[3][kMaxHist];
     double alpha[3][kMaxHist];
     double ys[3][kMaxHist], yy[3][kMaxHist];  // curvature of each slot's pair when it was formed
     double gamma[3];
-    double coefA[3], coefB[3];  // scratch coefficients for the next axpy
+    double coefA[3], coefB[3];  // coefficients for the next pass
     double dots[12];
     double pair[12];            // y.s, y.y, s.g, s.s of the newest pair
 };
@@ -366,59 +338,129 @@ struct LbOrder {
     int slot[kMaxHist];
 };
 
-// mode 0: newest pair formed: rho_k = 1/(y.s), first-loop alpha_k = rho_k (s_k.q) with q = g;
-//         with `guard`, a pair whose y.s <= 0 (no positive curvature along s) gets rho = 0 and so
-//         takes no part in either loop
-// mode 1: alpha_l = rho_l (s_l.q) from dots[0..2]
-// mode 3: beta = rho_l (y_l.r) from dots; coefB = alpha_l - beta
-__global__ void k_lb_scalar(LbScalars *S, int mode, int slot, int guard)
+// After the newest pair, o.slot[0]: rho = 1/(y.s), first-loop alpha = rho (s.q) with q = g; with
+// `guard`, a pair whose y.s <= 0 (no positive curvature along s) gets rho = 0 and so takes no part
+// in either loop.  And the scaling of the initial matrix, coefA = gamma = (s.y)/(y.y) of the newest
+// pair (src/main.c:622-655); with `guard`, of the newest pair with positive curvature, without one
+// |s| / |y| of the newest pair (a step as long as the last one, along the gradient).
+__device__ __forceinline__ void lb_pair_scalars(LbScalars *S, const LbOrder &o, int guard, int p)
 {
-    if (threadIdx.x != 0) return;
-    for (int p = 0; p < 3; p++) {
-        if (mode == 0) {
-            S->ys[p][slot] = S->pair[p];
-            S->yy[p][slot] = S->pair[3 + p];
-            S->rho[p][slot] = (guard && !(S->pair[p] > 0.0)) ? 0.0 : 1.0 / S->pair[p];
-            S->alpha[p][slot] = S->rho[p][slot] * S->pair[6 + p];
-            S->coefB[p] = -S->alpha[p][slot];
-        } else if (mode == 1) {
-            S->alpha[p][slot] = S->rho[p][slot] * S->dots[p];
-            S->coefB[p] = -S->alpha[p][slot];
-        } else {
-            double beta = S->rho[p][slot] * S->dots[p];
-            S->coefB[p] = S->alpha[p][slot] - beta;
-        }
-    }
-}
-
-// Scaling of the initial matrix, coefA = gamma = (s.y)/(y.y) of the newest pair (src/main.c:622-655).
-// With `guard`: of the newest pair with positive curvature; without one, |s| / |y| of the newest
-// pair (a step as long as the last one, along the gradient).
-__global__ void k_lb_gamma(LbScalars *S, LbOrder o, int guard)
-{
-    if (threadIdx.x != 0) return;
-    for (int p = 0; p < 3; p++) {
-        double gam = S->pair[p] / S->pair[3 + p];
-        if (guard) {
-            gam = sqrt(S->pair[9 + p] / S->pair[3 + p]);
-            for (int a = 0; a < o.n; a++) {
-                const int l = o.slot[a];
-                if (S->ys[p][l] > 0.0) {
-                    gam = S->ys[p][l] / S->yy[p][l];
-                    break;
-                }
+    const int slot = o.slot[0];
+    const double ys = S->pair[p], yy = S->pair[3 + p];
+    S->ys[p][slot] = ys;
+    S->yy[p][slot] = yy;
+    const double rho = (guard && !(ys > 0.0)) ? 0.0 : 1.0 / ys;
+    S->rho[p][slot] = rho;
+    S->alpha[p][slot] = rho * S->pair[6 + p];
+    S->coefB[p] = -S->alpha[p][slot];
+    double gam = ys / yy;
+    if (guard) {
+        gam = sqrt(S->pair[9 + p] / yy);
+        for (int a = 0; a < o.n; a++) {
+            const int l = o.slot[a];
+            if (S->ys[p][l] > 0.0) {
+                gam = S->ys[p][l] / S->yy[p][l];
+                break;
             }
         }
-        S->gamma[p] = gam;
-        S->coefA[p] = gam;
     }
+    S->gamma[p] = gam;
+    S->coefA[p] = gam;
 }
 
-// First-iteration scale 1/|g| (src/main.c:551-561).
-__global__ void k_lb_inv_norm(LbScalars *S)
+// s_k = m - m_back, y_k = g - g_back (3 parameters), the dots y.s, y.y, s.g, s.s and the scalars
+// after them; then m_back = m, g_back = g (src/main.c:683-688).
+template <typename T>
+__global__ void __launch_bounds__(kRedThreads) k_lb_pair(Tri<T> s, Tri<T> y, CTri<T> m, Tri<T> mb, CTri<T> g, Tri<T> gb,
+                                                         long n, DotScratch ds, LbScalars *S, LbOrder o, int guard)
 {
-    if (threadIdx.x != 0) return;
-    for (int p = 0; p < 3; p++) S->coefA[p] = 1.0 / sqrt(S->dots[p]);
+    using P = Pack<T>;
+    double v[4][3] = {};
+    for (long i = P::N * (blockIdx.x * (long)blockDim.x + threadIdx.x); i < n; i += P::N * (long)gridDim.x * blockDim.x)
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+            const P mv = P::get(m.p[p] + i), mo = P::get(mb.p[p] + i), gv = P::get(g.p[p] + i), go = P::get(gb.p[p] + i);
+            P sv, yv;
+#pragma unroll
+            for (int q = 0; q < P::N; q++) {
+                sv.v[q] = mv.v[q] - mo.v[q];
+                yv.v[q] = gv.v[q] - go.v[q];
+                const double sd = sv.v[q], yd = yv.v[q];
+                v[0][p] += yd * sd;
+                v[1][p] += yd * yd;
+                v[2][p] += sd * (double)gv.v[q];
+                v[3][p] += sd * sd;
+            }
+            sv.put(s.p[p] + i);
+            yv.put(y.p[p] + i);
+            mv.put(mb.p[p] + i);
+            gv.put(gb.p[p] + i);
+        }
+    reduce_last_block(v, ds, S->pair, [&](int p) { lb_pair_scalars(S, o, guard, p); });
+}
+
+// m_back = m, g_back = g and 1/|g| (src/main.c:551-561) into coefA.
+template <typename T>
+__global__ void __launch_bounds__(kRedThreads) k_lb_first(CTri<T> m, Tri<T> mb, CTri<T> g, Tri<T> gb, long n, DotScratch ds,
+                                                          LbScalars *S)
+{
+    using P = Pack<T>;
+    double v[1][3] = {};
+    for (long i = P::N * (blockIdx.x * (long)blockDim.x + threadIdx.x); i < n; i += P::N * (long)gridDim.x * blockDim.x)
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+            P::get(m.p[p] + i).put(mb.p[p] + i);
+            const P gv = P::get(g.p[p] + i);
+            gv.put(gb.p[p] + i);
+#pragma unroll
+            for (int q = 0; q < P::N; q++) v[0][p] += (double)gv.v[q] * (double)gv.v[q];
+        }
+    reduce_last_block(v, ds, S->dots, [&](int p) { S->coefA[p] = 1.0 / sqrt(S->dots[p]); });
+}
+
+// One pass of a loop: x := src + coefB u (per-parameter scalars, FP64) [GAMMA: then times coefA], the
+// dots next.x of slot `slot`, and the scalars after them:
+//  LB_FIRST (first loop): alpha = rho (s.q), coefB = -alpha
+//  LB_SECOND: beta = rho (y.r), coefB = alpha - beta
+//  LB_LAST: no dots
+enum { LB_FIRST, LB_SECOND, LB_LAST };
+template <typename T, int AFTER, bool GAMMA>
+__global__ void __launch_bounds__(kRedThreads) k_lb_axpy_dot(Tri<T> x, CTri<T> src, CTri<T> u, CTri<T> next, long n,
+                                                             DotScratch ds, LbScalars *S, int slot)
+{
+    using P = Pack<T>;
+    double v[1][3] = {};
+    double k1[3], gam[3];
+#pragma unroll
+    for (int p = 0; p < 3; p++) {
+        k1[p] = S->coefB[p];
+        gam[p] = GAMMA ? S->coefA[p] : 1.0;
+    }
+    for (long i = P::N * (blockIdx.x * (long)blockDim.x + threadIdx.x); i < n; i += P::N * (long)gridDim.x * blockDim.x)
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+            P xv = P::get(src.p[p] + i);
+            const P uv = P::get(u.p[p] + i);
+            P nv;
+            if (AFTER != LB_LAST) nv = P::get(next.p[p] + i);
+#pragma unroll
+            for (int q = 0; q < P::N; q++) {
+                xv.v[q] = (T)((double)xv.v[q] + k1[p] * (double)uv.v[q]);
+                if (GAMMA) xv.v[q] = (T)(gam[p] * (double)xv.v[q]);
+                if (AFTER != LB_LAST) v[0][p] += (double)nv.v[q] * (double)xv.v[q];
+            }
+            xv.put(x.p[p] + i);
+        }
+    if (AFTER != LB_LAST)
+        reduce_last_block(v, ds, S->dots, [&](int p) {
+            const double d = S->rho[p][slot] * S->dots[p];
+            if (AFTER == LB_FIRST) {
+                S->alpha[p][slot] = d;
+                S->coefB[p] = -d;
+            } else {
+                S->coefB[p] = S->alpha[p][slot] - d;
+            }
+        });
 }
 
 // v -= a_p * g * coefA_p below the layer, v_hor >= v_nmo (src/parallelcalls.cu:273-286).
@@ -426,9 +468,10 @@ template <typename T>
 __global__ void k_first_update(T *vh, T *vp, T *vn, const T *gh, const T *gp, const T *gn, const LbScalars *S,
                                float a_hor, float a_po, float a_nmo, int nx, int nz, int mpitch)
 {
-    long n = (long)nx * (nz - kLayer - 1);
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
-        long iz = kLayer + 1 + k / nx, ix = k % nx, i = iz * mpitch + ix;
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ix >= nx) return;
+    for (int iz = kLayer + 1 + blockIdx.y; iz < nz; iz += gridDim.y) {
+        const long i = (long)iz * mpitch + ix;
         vp[i] = vp[i] - (T)(a_po * (gp[i] * S->coefA[1]));
         T vnn = vn[i] - (T)(a_nmo * (gn[i] * S->coefA[2]));
         T vhn = vh[i] - (T)(a_hor * (gh[i] * S->coefA[0]));
@@ -442,13 +485,13 @@ __global__ void k_first_update(T *vh, T *vp, T *vn, const T *gh, const T *gp, co
 template <typename T>
 __global__ void k_lb_slope(CTri<T> g, CTri<T> r, int nx, int nz, int mpitch, DotScratch ds, double *out)
 {
-    double v[4][3] = {};
+    double v[1][3] = {};
     const long n = (long)nx * (nz - kLayer - 1);
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
         const long iz = kLayer + 1 + k / nx, ix = k % nx, i = iz * mpitch + ix;
         for (int p = 0; p < 3; p++) v[0][p] += (double)g.p[p][i] * r.p[p][i];
     }
-    reduce_last_block(v, 1, ds, out);
+    reduce_last_block(v, ds, out, [](int) {});
 }
 
 // Trial model (src/parallelcalls.cu:343-404) for all three parameters.
@@ -457,9 +500,10 @@ __global__ void k_lb_update(T *vh, T *vp, T *vn, const T *bh, const T *bp, const
                             const T *rp, const T *rn, float av, float ad, float ae, int fmin, int fmax,
                             int nx, int nz, int mpitch)
 {
-    long n = (long)nx * (nz - kLayer - 1);
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
-        long iz = kLayer + 1 + k / nx, ix = k % nx, i = iz * mpitch + ix;
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ix >= nx) return;
+    for (int iz = kLayer + 1 + blockIdx.y; iz < nz; iz += gridDim.y) {
+        const long i = (long)iz * mpitch + ix;
         T p = bp[i] - (T)av * rp[i];
         if (fmax == 1 && p > T(3.5e6)) p = T(3.5e6);
         if (fmin == 1 && p < T(1.8e6)) p = T(1.8e6);
@@ -1003,7 +1047,9 @@ template <typename T> struct Ctx : CtxBase {
         TRY(alloc(&ds.counter, 1));
         TRY(cudaMemsetAsync(ds.counter, 0, sizeof(unsigned), st));
         TRY(cudaMemsetAsync(lbs, 0, sizeof(LbScalars), st));
-        for (T *p : {vh, vp, vn, mh, mp, mn}) TRY(cudaMemsetAsync(p, 0, mslot * sizeof(T), st));
+        // padding of the model's rows included: the optimizer's sums run over it
+        for (T *p : {vh, vp, vn, mh, mp, mn, grad[0], grad[1], grad[2]})
+            TRY(cudaMemsetAsync(p, 0, mslot * sizeof(T), st));
         int rcc = cpml_table();
         if (rcc) return rcc;
         TRY_LAUNCH();
@@ -2390,9 +2436,10 @@ template <typename T> struct Ctx : CtxBase {
 
     // ---------------------------------------------------------------- L-BFGS
 
+    // 256 columns a block, a row at a time
+    dim3 row_grid() const { return dim3((nx + 255) / 256, std::min(nz, 65535)); }
     Tri<T> tri(T *const (&a)[3]) const { Tri<T> t; for (int k = 0; k < 3; k++) t.p[k] = a[k]; return t; }
     CTri<T> ctri(T *const (&a)[3]) const { CTri<T> t; for (int k = 0; k < 3; k++) t.p[k] = a[k]; return t; }
-    CTri<T> cnull() const { CTri<T> t; for (int k = 0; k < 3; k++) t.p[k] = nullptr; return t; }
 
     int copy3(T *const (&dst)[3], T *const (&src)[3])
     {
@@ -2404,16 +2451,13 @@ template <typename T> struct Ctx : CtxBase {
     {
         if (!have_grad || !have_model) return FWI_ERR_STATE;
         T *m3[3] = {vh, vp, vn};
-        int rc;
-        if ((rc = copy3(mb, m3)) || (rc = copy3(gb, grad))) return rc;
         have_back = true;
         // |g|^2 over the whole grid (src/main.c:551-559), in FP64
-        k_lb_copy_dot<T><<<red_blocks, kRedThreads, 0, st>>>(tri(q), ctri(grad), ctri(grad), mslot, ds, lbs->dots);
-        k_lb_inv_norm<<<1, 32, 0, st>>>(lbs);
-        k_first_update<T><<<eg((long)nx * nz), 256, 0, st>>>(vh, vp, vn, grad[0], grad[1], grad[2], lbs, a_hor,
-                                                                   a_po, a_nmo, nx, nz, mpitch);
+        k_lb_first<T><<<red_blocks, kRedThreads, 0, st>>>(ctri(m3), tri(mb), ctri(grad), tri(gb), mslot, ds, lbs);
+        k_first_update<T><<<row_grid(), 256, 0, st>>>(vh, vp, vn, grad[0], grad[1], grad[2], lbs, a_hor, a_po, a_nmo, nx,
+                                                      nz, mpitch);
         TRY_LAUNCH();
-        launches += 3;
+        launches += 2;
         models_dirty = true;
         hist_count = 0;
         hist_next = 0;
@@ -2445,52 +2489,36 @@ template <typename T> struct Ctx : CtxBase {
         const int k = hist_next % m;
         T *sk[3] = {hs[k][0], hs[k][1], hs[k][2]}, *yk[3] = {hy[k][0], hy[k][1], hy[k][2]};
         T *m3[3] = {vh, vp, vn};
-        k_lb_pair<T><<<red_blocks, kRedThreads, 0, st>>>(tri(sk), tri(yk), ctri(m3), ctri(mb), ctri(grad), ctri(gb),
-                                                         mslot, ds, lbs->pair);
         hist_next = (hist_next + 1) % m;
         hist_count = std::min(hist_count + 1, m);
-        // order newest .. oldest
-        std::vector<int> order;
-        for (int a = 0; a < hist_count; a++) order.push_back(((hist_next - 1 - a) % m + m) % m);
-        // first loop; q = g and rho_k, alpha_k of the newest pair
-        int rcq = copy3(q, grad);
-        if (rcq) return rcq;
-        k_lb_scalar<<<1, 32, 0, st>>>(lbs, 0, order[0], lb_guard);
-        // rho of the older slots persists from when they were formed
-        for (size_t a = 0; a < order.size(); a++) {
-            const int l = order[a];
-            T *yl[3] = {hy[l][0], hy[l][1], hy[l][2]};
-            if (a > 0) k_lb_scalar<<<1, 32, 0, st>>>(lbs, 1, l, lb_guard);
-            const bool has_next = a + 1 < order.size();
-            const int ln = has_next ? order[a + 1] : l;
-            T *sn[3] = {hs[ln][0], hs[ln][1], hs[ln][2]};
-            k_lb_axpy_dot<T><<<red_blocks, kRedThreads, 0, st>>>(tri(q), ctri(yl), nullptr, lbs->coefB, ctri(sn),
-                                                                 has_next ? 1 : 0, mslot, ds, lbs->dots);
+        LbOrder lo{};  // newest .. oldest
+        lo.n = hist_count;
+        for (int a = 0; a < lo.n; a++) lo.slot[a] = ((hist_next - 1 - a) % m + m) % m;
+        k_lb_pair<T><<<red_blocks, kRedThreads, 0, st>>>(tri(sk), tri(yk), ctri(m3), tri(mb), ctri(grad), tri(gb), mslot,
+                                                         ds, lbs, lo, lb_guard);
+        // first loop, from q = g (rho of the older slots persists from when they were formed); its last
+        // pass makes r = gamma q
+        for (int a = 0; a < lo.n; a++) {
+            const int l = lo.slot[a];
+            const CTri<T> src = a == 0 ? ctri(grad) : ctri(q);
+            if (a + 1 < lo.n)
+                k_lb_axpy_dot<T, LB_FIRST, false><<<red_blocks, kRedThreads, 0, st>>>(
+                    tri(q), src, ctri(hy[l]), ctri(hs[lo.slot[a + 1]]), mslot, ds, lbs, lo.slot[a + 1]);
+            else
+                k_lb_axpy_dot<T, LB_SECOND, true><<<red_blocks, kRedThreads, 0, st>>>(tri(r), src, ctri(hy[l]), ctri(hy[l]),
+                                                                                      mslot, ds, lbs, l);
         }
-        // r = gamma q; then the second loop oldest .. newest
-        LbOrder lo{};
-        lo.n = (int)order.size();
-        for (int a = 0; a < lo.n; a++) lo.slot[a] = order[a];
-        k_lb_gamma<<<1, 32, 0, st>>>(lbs, lo, lb_guard);
-        int first = order.back();
-        T *y0[3] = {hy[first][0], hy[first][1], hy[first][2]};
-        rcq = copy3(r, q);
-        if (rcq) return rcq;
-        k_lb_axpy_dot<T><<<red_blocks, kRedThreads, 0, st>>>(tri(r), cnull(), lbs->coefA, nullptr, ctri(y0), 1, mslot,
-                                                             ds, lbs->dots);
-        for (int a = (int)order.size() - 1; a >= 0; a--) {
-            const int l = order[a];
-            T *sl[3] = {hs[l][0], hs[l][1], hs[l][2]};
-            k_lb_scalar<<<1, 32, 0, st>>>(lbs, 3, l, lb_guard);
-            const bool has_next = a > 0;
-            const int ln = has_next ? order[a - 1] : l;
-            T *yn[3] = {hy[ln][0], hy[ln][1], hy[ln][2]};
-            k_lb_axpy_dot<T><<<red_blocks, kRedThreads, 0, st>>>(tri(r), ctri(sl), nullptr, lbs->coefB, ctri(yn),
-                                                                 has_next ? 1 : 0, mslot, ds, lbs->dots);
+        // second loop, oldest .. newest
+        for (int a = lo.n - 1; a >= 0; a--) {
+            const int l = lo.slot[a];
+            if (a > 0)
+                k_lb_axpy_dot<T, LB_SECOND, false><<<red_blocks, kRedThreads, 0, st>>>(
+                    tri(r), ctri(r), ctri(hs[l]), ctri(hy[lo.slot[a - 1]]), mslot, ds, lbs, lo.slot[a - 1]);
+            else
+                k_lb_axpy_dot<T, LB_LAST, false><<<red_blocks, kRedThreads, 0, st>>>(tri(r), ctri(r), ctri(hs[l]), ctri(r),
+                                                                                     mslot, ds, lbs, l);
         }
         TRY_LAUNCH();
-        // the model and gradient this direction starts from (src/main.c:683-688)
-        if ((rc = copy3(mb, m3)) || (rc = copy3(gb, grad))) return rc;
         have_dir = true;
         if (stats) {
             LbScalars h;
@@ -2498,7 +2526,7 @@ template <typename T> struct Ctx : CtxBase {
             TRY(cudaStreamSynchronize(st));
             for (int p = 0; p < 3; p++) {
                 stats[p] = h.gamma[p];
-                stats[3 + p] = h.rho[p][order[0]];
+                stats[3 + p] = h.rho[p][lo.slot[0]];
                 stats[6 + p] = h.pair[p];      // y.s of the newest pair
                 stats[9 + p] = h.pair[3 + p];  // y.y of the newest pair
             }
@@ -2526,8 +2554,8 @@ template <typename T> struct Ctx : CtxBase {
     {
         if (!have_back) return FWI_ERR_STATE;
         // av, ad, ae pair with (v_po, v_nmo, v_hor) as update_LBFGS does (src/main.c:693)
-        k_lb_update<T><<<eg((long)nx * nz), 256, 0, st>>>(vh, vp, vn, mb[0], mb[1], mb[2], r[0], r[1], r[2], av,
-                                                                ad, ae, fmin, fmax, nx, nz, mpitch);
+        k_lb_update<T><<<row_grid(), 256, 0, st>>>(vh, vp, vn, mb[0], mb[1], mb[2], r[0], r[1], r[2], av, ad, ae, fmin,
+                                                   fmax, nx, nz, mpitch);
         TRY_LAUNCH();
         launches++;
         models_dirty = true;
