@@ -315,11 +315,61 @@ template <typename T> struct alignas(16) Pack {
     __device__ __forceinline__ void put(T *p) const { *reinterpret_cast<Pack *>(p) = *this; }
 };
 
-// The passes of the L-BFGS recursion below are bound by the FP64 pipe (64 cycles a warp instruction
-// on an SM quarter; the sums and coefficients are FP64) and, per pass, by the launch and the last
-// block's tail.  So: no FP64 multiplication that an operand of 1 or 0 makes idle, copies made by the
-// pass that has the values in registers, scalar bookkeeping in the last block of the reduction that
-// feeds it.  On a 2009 x 809 model, first step and 5 directions and updates: 4.9 -> 1.5 ms.
+// The passes of the L-BFGS recursion below: sums and coefficients are FP64, whose pipe takes 64 cycles
+// a warp instruction on an SM quarter, conversions from and to FP32 included (an axpy with a dot, 7 such
+// operations a value, was bound by them: 75 us for 3 x 1.6 M values).  So: FP32 widens by integer
+// operations, x + k u is rounded from error-free FP32 parts, no FP64 operation by 1 or 0; copies made by
+// the pass that has the values, scalar steps by the last block of the reduction that feeds them.
+// First step and 5 directions and updates on 2009 x 809: 4.90 ms before, 3.37 with FP64
+// conversions in 2 blocks an SM, 1.9 now.
+
+// The rare cases, out of line: as branches the compiler would run their FP64 operations for every value.
+__device__ __noinline__ double widen_any(float v) { return (double)v; }
+__device__ __noinline__ float axpy_any(float x, float u, double k) { return (float)((double)x + k * (double)u); }
+
+__device__ __forceinline__ double widen(double v) { return v; }
+// Exact; all but normal values and zeros (rare) by the conversion.
+__device__ __forceinline__ double widen(float v)
+{
+    const unsigned u = __float_as_uint(v), e = u & 0x7f800000u;
+    if (e == 0x7f800000u || (e == 0 && (u << 1) != 0)) return widen_any(v);
+    const unsigned hi = (u & 0x80000000u) | (e ? ((u & 0x7fffffffu) >> 3) + 0x38000000u : 0u);
+    return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+// An FP64 coefficient, for FP32 operands in two parts (48 bits) when it lies well inside FP32's range.
+template <typename T> struct LbCoef {
+    double k;
+    __device__ __forceinline__ explicit LbCoef(double k_) : k(k_) {}
+    __device__ __forceinline__ T axpy(T x, T u) const { return x + k * u; }
+    __device__ __forceinline__ T scale(T x) const { return k * x; }
+};
+template <> struct LbCoef<float> {
+    double k;
+    float h, l;
+    bool parts;
+    __device__ __forceinline__ explicit LbCoef(double k_) : k(k_), h((float)k_)
+    {
+        l = (float)(k - (double)h);
+        parts = fabs(k) < 1e30 && (fabs(k) > 1e-20 || k == 0.0);
+    }
+    // x + k u rounded once, to within 2^-20 of a last place of FP64's value: the product and the sum
+    // with their exact errors (fused multiply-add; Knuth's two-sum), then one rounding.  Where a part
+    // could underflow or overflow, in FP64.
+    __device__ __forceinline__ float axpy(float x, float u) const
+    {
+        const float p = h * u, e = __fmaf_rn(h, u, -p), s = x + p, t = s - x;
+        const float r = s + (((x - (s - t)) + (p - t)) + __fmaf_rn(l, u, e));
+        if (parts && fabsf(r) <= 3e38f && (fmaxf(fabsf(p), fabsf(x)) > 0x1p-70f || u == 0.f)) return r;
+        return axpy_any(x, u, k);
+    }
+    __device__ __forceinline__ float scale(float x) const
+    {
+        const float p = h * x, r = p + __fmaf_rn(l, x, __fmaf_rn(h, x, -p));
+        if (parts && fabsf(r) <= 3e38f && (fabsf(p) > 0x1p-70f || x == 0.f)) return r;
+        return axpy_any(0.f, x, k);
+    }
+};
 
 // Scalars of the two-loop recursion.
 struct LbScalars {
@@ -385,10 +435,10 @@ __global__ void __launch_bounds__(kRedThreads) k_lb_pair(Tri<T> s, Tri<T> y, CTr
             for (int q = 0; q < P::N; q++) {
                 sv.v[q] = mv.v[q] - mo.v[q];
                 yv.v[q] = gv.v[q] - go.v[q];
-                const double sd = sv.v[q], yd = yv.v[q];
+                const double sd = widen(sv.v[q]), yd = widen(yv.v[q]);
                 v[0][p] += yd * sd;
                 v[1][p] += yd * yd;
-                v[2][p] += sd * (double)gv.v[q];
+                v[2][p] += sd * widen(gv.v[q]);
                 v[3][p] += sd * sd;
             }
             sv.put(s.p[p] + i);
@@ -413,7 +463,10 @@ __global__ void __launch_bounds__(kRedThreads) k_lb_first(CTri<T> m, Tri<T> mb, 
             const P gv = P::get(g.p[p] + i);
             gv.put(gb.p[p] + i);
 #pragma unroll
-            for (int q = 0; q < P::N; q++) v[0][p] += (double)gv.v[q] * (double)gv.v[q];
+            for (int q = 0; q < P::N; q++) {
+                const double w = widen(gv.v[q]);
+                v[0][p] += w * w;
+            }
         }
     reduce_last_block(v, ds, S->dots, [&](int p) { S->coefA[p] = 1.0 / sqrt(S->dots[p]); });
 }
@@ -430,12 +483,8 @@ __global__ void __launch_bounds__(kRedThreads) k_lb_axpy_dot(Tri<T> x, CTri<T> s
 {
     using P = Pack<T>;
     double v[1][3] = {};
-    double k1[3], gam[3];
-#pragma unroll
-    for (int p = 0; p < 3; p++) {
-        k1[p] = S->coefB[p];
-        gam[p] = GAMMA ? S->coefA[p] : 1.0;
-    }
+    const LbCoef<T> k1[3] = {LbCoef<T>(S->coefB[0]), LbCoef<T>(S->coefB[1]), LbCoef<T>(S->coefB[2])};
+    const LbCoef<T> gam[3] = {LbCoef<T>(S->coefA[0]), LbCoef<T>(S->coefA[1]), LbCoef<T>(S->coefA[2])};
     for (long i = P::N * (blockIdx.x * (long)blockDim.x + threadIdx.x); i < n; i += P::N * (long)gridDim.x * blockDim.x)
 #pragma unroll
         for (int p = 0; p < 3; p++) {
@@ -445,9 +494,9 @@ __global__ void __launch_bounds__(kRedThreads) k_lb_axpy_dot(Tri<T> x, CTri<T> s
             if (AFTER != LB_LAST) nv = P::get(next.p[p] + i);
 #pragma unroll
             for (int q = 0; q < P::N; q++) {
-                xv.v[q] = (T)((double)xv.v[q] + k1[p] * (double)uv.v[q]);
-                if (GAMMA) xv.v[q] = (T)(gam[p] * (double)xv.v[q]);
-                if (AFTER != LB_LAST) v[0][p] += (double)nv.v[q] * (double)xv.v[q];
+                xv.v[q] = k1[p].axpy(xv.v[q], uv.v[q]);
+                if (GAMMA) xv.v[q] = gam[p].scale(xv.v[q]);
+                if (AFTER != LB_LAST) v[0][p] += widen(nv.v[q]) * widen(xv.v[q]);
             }
             xv.put(x.p[p] + i);
         }
@@ -585,6 +634,7 @@ struct CtxBase {
     int last_cuda = 0;
     int n_sm = 1;        // streaming multiprocessors of the context's device
     int red_blocks = 2;  // blocks of the reduction kernels: 2 per SM
+    int lb_blocks = 3;   // of the L-BFGS passes: 3 per SM (5 pairs, 2009 x 809: 391 us; 2: 432, 4: 412, 8: 546)
     unsigned eg(long n) const { return elt_grid(n, n_sm); }
     float timing[4] = {0, 0, 0, 0};
     long launches = 0;
@@ -960,6 +1010,7 @@ template <typename T> struct Ctx : CtxBase {
         TRY(cudaSetDevice(cfg.device));
         TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, cfg.device));
         red_blocks = 2 * n_sm;
+        lb_blocks = 3 * n_sm;
         if (const char *e = getenv("FWI_GRAPHS")) graphs = atoi(e) != 0;
         TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         for (auto &e : ev) TRY(cudaEventCreate(&e));
@@ -1043,7 +1094,7 @@ template <typename T> struct Ctx : CtxBase {
         for (T **p : {&mb[0], &mb[1], &mb[2], &gb[0], &gb[1], &gb[2], &q[0], &q[1], &q[2], &r[0], &r[1], &r[2]})
             TRY(alloc(p, mslot));
         TRY(alloc(&lbs, 1));
-        TRY(alloc(&ds.partial, (size_t)red_blocks * 12));
+        TRY(alloc(&ds.partial, (size_t)std::max(red_blocks, lb_blocks) * 12));
         TRY(alloc(&ds.counter, 1));
         TRY(cudaMemsetAsync(ds.counter, 0, sizeof(unsigned), st));
         TRY(cudaMemsetAsync(lbs, 0, sizeof(LbScalars), st));
@@ -2453,7 +2504,7 @@ template <typename T> struct Ctx : CtxBase {
         T *m3[3] = {vh, vp, vn};
         have_back = true;
         // |g|^2 over the whole grid (src/main.c:551-559), in FP64
-        k_lb_first<T><<<red_blocks, kRedThreads, 0, st>>>(ctri(m3), tri(mb), ctri(grad), tri(gb), mslot, ds, lbs);
+        k_lb_first<T><<<lb_blocks, kRedThreads, 0, st>>>(ctri(m3), tri(mb), ctri(grad), tri(gb), mslot, ds, lbs);
         k_first_update<T><<<row_grid(), 256, 0, st>>>(vh, vp, vn, grad[0], grad[1], grad[2], lbs, a_hor, a_po, a_nmo, nx,
                                                       nz, mpitch);
         TRY_LAUNCH();
@@ -2494,7 +2545,7 @@ template <typename T> struct Ctx : CtxBase {
         LbOrder lo{};  // newest .. oldest
         lo.n = hist_count;
         for (int a = 0; a < lo.n; a++) lo.slot[a] = ((hist_next - 1 - a) % m + m) % m;
-        k_lb_pair<T><<<red_blocks, kRedThreads, 0, st>>>(tri(sk), tri(yk), ctri(m3), tri(mb), ctri(grad), tri(gb), mslot,
+        k_lb_pair<T><<<lb_blocks, kRedThreads, 0, st>>>(tri(sk), tri(yk), ctri(m3), tri(mb), ctri(grad), tri(gb), mslot,
                                                          ds, lbs, lo, lb_guard);
         // first loop, from q = g (rho of the older slots persists from when they were formed); its last
         // pass makes r = gamma q
@@ -2502,20 +2553,20 @@ template <typename T> struct Ctx : CtxBase {
             const int l = lo.slot[a];
             const CTri<T> src = a == 0 ? ctri(grad) : ctri(q);
             if (a + 1 < lo.n)
-                k_lb_axpy_dot<T, LB_FIRST, false><<<red_blocks, kRedThreads, 0, st>>>(
+                k_lb_axpy_dot<T, LB_FIRST, false><<<lb_blocks, kRedThreads, 0, st>>>(
                     tri(q), src, ctri(hy[l]), ctri(hs[lo.slot[a + 1]]), mslot, ds, lbs, lo.slot[a + 1]);
             else
-                k_lb_axpy_dot<T, LB_SECOND, true><<<red_blocks, kRedThreads, 0, st>>>(tri(r), src, ctri(hy[l]), ctri(hy[l]),
+                k_lb_axpy_dot<T, LB_SECOND, true><<<lb_blocks, kRedThreads, 0, st>>>(tri(r), src, ctri(hy[l]), ctri(hy[l]),
                                                                                       mslot, ds, lbs, l);
         }
         // second loop, oldest .. newest
         for (int a = lo.n - 1; a >= 0; a--) {
             const int l = lo.slot[a];
             if (a > 0)
-                k_lb_axpy_dot<T, LB_SECOND, false><<<red_blocks, kRedThreads, 0, st>>>(
+                k_lb_axpy_dot<T, LB_SECOND, false><<<lb_blocks, kRedThreads, 0, st>>>(
                     tri(r), ctri(r), ctri(hs[l]), ctri(hy[lo.slot[a - 1]]), mslot, ds, lbs, lo.slot[a - 1]);
             else
-                k_lb_axpy_dot<T, LB_LAST, false><<<red_blocks, kRedThreads, 0, st>>>(tri(r), ctri(r), ctri(hs[l]), ctri(r),
+                k_lb_axpy_dot<T, LB_LAST, false><<<lb_blocks, kRedThreads, 0, st>>>(tri(r), ctri(r), ctri(hs[l]), ctri(r),
                                                                                      mslot, ds, lbs, l);
         }
         TRY_LAUNCH();
