@@ -21,7 +21,8 @@ BUILD = os.path.join(PKG, "_build")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libfwi_gb300.so")
 
-UNITS = ["compat.cu", "native.cu", "prop_f32.cu", "prop_resident.cu", "prop_f64.cu", "noalloc.cu"]
+UNITS = ["compat.cu", "native.cu", "prop_f32.cu", "prop_resident.cu", "prop_resident_ref.cu",
+         "prop_f64.cu", "noalloc.cu"]
 # compat.cu reproduces the reference's arithmetic operation for operation: no multiply-add contraction
 UNIT_FLAGS = {"compat.cu": ["--fmad=false"]}
 C_UNITS = ["driver.c"]  # host C over the C-ABI

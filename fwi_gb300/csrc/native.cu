@@ -1351,9 +1351,9 @@ template <typename T> struct Ctx : CtxBase {
         if (sizeof(T) != 4 || !use_tma) return false;
         if (const char *e = getenv("FWI_CLUSTER"))
             if (atoi(e) == 0) return false;
-        const bool exact = cfg.mode == FWI_MODE_EXACT, ckpt = want_grad && cfg.store == FWI_STORE_CHECKPOINT;
+        const bool ckpt = want_grad && cfg.store == FWI_STORE_CHECKPOINT;
         const bool full = want_grad && cfg.store == FWI_STORE_FULL;
-        if (want_grad && !full && !(ckpt && exact)) return false;
+        if (want_grad && !full && !ckpt) return false;
         const int at_once = cluster_path(nxm);
         if ((long)nxm * nz <= 12000 && at_once && (int)bs.size() <= at_once) return false;
         long points = 0;
@@ -1366,7 +1366,7 @@ template <typename T> struct Ctx : CtxBase {
         const size_t lim = fwd || nxm <= 640 ? fwi::resident_smem_limit() : 0;
         if (!lim) return false;
         if (fwd) run.fwd = resident_sets(w, 0, lim);
-        if (exact && (full ? nxm <= 640 : ckpt && run.fwd)) run.adj = resident_sets(w, (int)store_elem(), lim);
+        if (full ? nxm <= 640 : ckpt && run.fwd) run.adj = resident_sets(w, (int)store_elem(), lim);
         if (run.adj && nxm > 400 && run.adj->size() > 1) run.adj = nullptr;
         if (ckpt && !run.adj) run.fwd = nullptr;
         if (!run.any()) return false;
@@ -1444,6 +1444,7 @@ template <typename T> struct Ctx : CtxBase {
                          int img_base)
     {
         if constexpr (sizeof(T) == 4) {
+            const bool exact = cfg.mode == FWI_MODE_EXACT;
             for (const fwi::ResidentSet &set : sets) {
                 fwi::ResAdjArgs a{};
                 unsigned tag = 0;
@@ -1455,7 +1456,7 @@ template <typename T> struct Ctx : CtxBase {
                 a.img_base = img_base;
                 a.x = res_x;
                 a.tag0 = tag - (unsigned)j0;
-                TRY(fwi::launch_resident_adjoint(b, set, a, st));
+                TRY(exact ? fwi::launch_resident_adjoint(b, set, a, st) : fwi::launch_resident_ref_adjoint(b, set, a, st));
                 launches++;
             }
         }
@@ -1903,13 +1904,18 @@ template <typename T> struct Ctx : CtxBase {
                     // segments', which the forward kept), then the adjoint iterations that image in it
                     Batch<T> rb = bf;
                     rb.rec = obs;  // `rec` holds the residuals now
+                    const int lag = exact ? 0 : 1;
+                    int j = 0;
                     for (int seg = last_seg; seg >= 0; seg--) {
                         const int a = seg * ck_every, e = std::min(a + ck_every, ntb), h = seg & 1;
                         if (seg < first_direct) {
                             if ((rc = resident_forward(rb, *resident.fwd, nxm, ntb, a, e, a, ck_every, seg, 0))) return rc;
                             recompute_steps += e - a;
                         }
-                        if ((rc = resident_adjoint(b, *resident.adj, ntb, ntb - e, ntb - a, a - h * ck_every))) return rc;
+                        // (reference mode: an iteration images one step earlier, the last one none)
+                        const int j1 = seg > 0 ? ntb - lag - a : ntb;
+                        if (j1 > j && (rc = resident_adjoint(b, *resident.adj, ntb, j, j1, a - h * ck_every))) return rc;
+                        j = std::max(j, j1);
                     }
                 }
                 // one gradient slot per shot

@@ -229,6 +229,8 @@ struct ResAdjArgs;
 size_t resident_smem_limit();
 cudaError_t launch_resident_forward(const Batch<float> &b, const ResidentSet &set, const ResFwdArgs &a, cudaStream_t st);
 cudaError_t launch_resident_adjoint(const Batch<float> &b, const ResidentSet &set, const ResAdjArgs &a, cudaStream_t st);
+cudaError_t launch_resident_ref_adjoint(const Batch<float> &b, const ResidentSet &set, const ResAdjArgs &a,
+                                        cudaStream_t st);
 
 // Boundary storage (prop_boundary.cuh): ring length per shot, saving the
 // ring of step g, and the backward rebuild of the CPML-free region.

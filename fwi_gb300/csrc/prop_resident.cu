@@ -1,4 +1,5 @@
-// Launches of the resident path (prop_resident.cuh): one cooperative launch per set of shots.
+// Launches of the resident path (prop_resident.cuh): one cooperative launch per set of shots.  The
+// reference-mode adjoint's kernels are in prop_resident_ref.cu.
 #include <mutex>
 
 #include "prop_resident.cuh"
@@ -6,8 +7,6 @@
 namespace fwi {
 
 namespace {
-
-template <typename Args> using ResKernel = void (*)(Batch<float>, ResidentGrid, Args);
 
 template <int ST> ResKernel<ResFwdArgs> fwd_kernel(int pitch)
 {
@@ -20,49 +19,15 @@ template <int ST> ResKernel<ResFwdArgs> fwd_kernel(int pitch)
     default: return nullptr;
     }
 }
-template <int ST> ResKernel<ResAdjArgs> adj_kernel(int pitch)
-{
-    switch (pitch) {
-    case 96: return k_resident_adj<ST, 96>;
-    case 160: return k_resident_adj<ST, 160>;
-    case 224: return k_resident_adj<ST, 224>;
-    case 320: return k_resident_adj<ST, 320>;
-    case 400: return k_resident_adj<ST, 400>;
-    case 512: return k_resident_adj<ST, 512>;
-    case 640: return k_resident_adj<ST, 640>;
-    default: return nullptr;
-    }
-}
 ResKernel<ResFwdArgs> fwd_kernel(int store_type, int pitch)
 {
     return store_type == kStoreHalf ? fwd_kernel<kStoreHalf>(pitch)
            : store_type == kStoreBf16 ? fwd_kernel<kStoreBf16>(pitch) : fwd_kernel<kStoreNative>(pitch);
 }
-ResKernel<ResAdjArgs> adj_kernel(int store_type, int pitch)
-{
-    return store_type == kStoreHalf ? adj_kernel<kStoreHalf>(pitch)
-           : store_type == kStoreBf16 ? adj_kernel<kStoreBf16>(pitch) : adj_kernel<kStoreNative>(pitch);
-}
-
-// Cooperative: every CTA of the launch is resident before any of them waits on another.
-template <typename Args>
-cudaError_t launch(ResKernel<Args> k, const Batch<float> &b, const ResidentSet &set, const Args &a, cudaStream_t st)
-{
-    if (!k) return cudaErrorInvalidValue;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(set.grid.n);
-    cfg.blockDim = dim3(set.threads);
-    cfg.dynamicSmemBytes = set.smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, b, set.grid, a);
-}
 
 }  // namespace
+
+bool resident_allow_ref(int smem);  // prop_resident_ref.cu
 
 // Dynamic shared memory of a CTA on the current device (0: the kernels cannot run there): the
 // device's opt-in limit less their static shared memory; the function attributes are set once.
@@ -82,11 +47,8 @@ size_t resident_smem_limit()
     bool ok = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
               cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop && optin > 1024;
     const int lim = optin - 1024;
-    for (int st : {(int)kStoreNative, (int)kStoreHalf, (int)kStoreBf16}) {
-        for (int p : kResPitches)
-            for (const void *k : {(const void *)fwd_kernel(st, p), (const void *)adj_kernel(st, p)})
-                ok = ok && (!k || cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) == cudaSuccess);
-    }
+    ok = ok && res_allow([](int st, int p) { return fwd_kernel(st, p); }, lim) &&
+         res_allow([](int st, int p) { return res_adj_kernel<false>(st, p); }, lim) && resident_allow_ref(lim);
     if (!ok) cudaGetLastError();
     limit[dev] = ok ? (size_t)lim : 0;
     done[dev] = true;
@@ -95,12 +57,12 @@ size_t resident_smem_limit()
 
 cudaError_t launch_resident_forward(const Batch<float> &b, const ResidentSet &set, const ResFwdArgs &a, cudaStream_t st)
 {
-    return launch(fwd_kernel(b.store_type, set.pitch), b, set, a, st);
+    return res_launch(fwd_kernel(b.store_type, set.pitch), b, set, a, st);
 }
 
 cudaError_t launch_resident_adjoint(const Batch<float> &b, const ResidentSet &set, const ResAdjArgs &a, cudaStream_t st)
 {
-    return launch(adj_kernel(b.store_type, set.pitch), b, set, a, st);
+    return res_launch(res_adj_kernel<false>(b.store_type, set.pitch), b, set, a, st);
 }
 
 }  // namespace fwi

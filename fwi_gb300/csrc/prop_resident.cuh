@@ -652,9 +652,15 @@ k_resident_fwd(const __grid_constant__ Batch<float> b, const __grid_constant__ R
     }
 }
 
-// ------------------------------------------------------------------ exact adjoint
+// ------------------------------------------------------------------ adjoint
 
-template <int ST, int PT>
+// REF: the reference's adjoint, whose CPML is the forward's, applied to the model-weighted fields
+// (src/parallelcalls.cu:179-243).  Its four psi and four zeta are linear in them and pairs share their
+// coefficients and enter the update as sums, so that the sums are advanced: psi_x' = b psi_x + a Dx u_x
+// with u_x = v_hor lambda_P + v_nmo lambda_F (and z, u_z = v_po (lambda_P + lambda_F)): the forward's two psi
+// and two zeta.  Iteration j images step nt - 2 - j (the exact adjoint: nt - 1 - j).
+
+template <int ST, int PT, bool REF>
 __global__ void __launch_bounds__(res_shape(PT).threads, 1)
 k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ ResidentGrid grid,
                const __grid_constant__ ResAdjArgs a)
@@ -664,7 +670,8 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
     using Img = ResImage<Cd>;
     constexpr int R = res_shape(PT).adj_rows;
     constexpr int OWN = kResAdjOwn;                 // own arrays: u_x (two levels), v_hor, v_po, v_nmo, three gradients
-    constexpr int WB = kResSide, SD = kResAdjSide;  // side arrays: Y_x, Z_x, a Y_x, u_x at layer points, -Dx(a Y_x)
+    constexpr int WB = kResSide, SD = kResAdjSide;  // side arrays: Y_x, Z_x, a Y_x, u_x at layer points,
+                                                  // -Dx(a Y_x); REF: psi_x, zeta_x, what they add to Dxx u_x
     extern __shared__ __align__(16) float csm[];
     __shared__ int dead;
     const DevShot sh = b.shots[grid.shot[blockIdx.x]];
@@ -694,7 +701,7 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
         float *const o = pO + rr * OWN * PT;
         float2 ux = fma(ld2(o + 2 * PT), lp, mul(ld2(o + 4 * PT), lf)), uz = mul(ld2(o + 3 * PT), add(lp, lf));
         const int r = r0 + rr;
-        const bool zl = B.bottom && B.iz0 + r >= B.zb;
+        const bool zl = !REF && B.bottom && B.iz0 + r >= B.zb;
         if (zl) {
             float *const z_ = S.zo + r * 2 * PT + ix;
             float2 z = ld2(z_);
@@ -704,7 +711,7 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
             }
             uz = fma(both(S.az[r]), z, uz);
         }
-        if (B.side) {
+        if (!REF && B.side) {
             float *const ps = pS + rr * SD * WB;
             if (lay0 || lay1) {
                 float2 z = ld2(ps + WB);
@@ -773,22 +780,42 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
             }
         if constexpr (STAGE) asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (a.j0 < j1) stage_images(a.ntb - 1 - a.j0);
+    constexpr int LAG = REF ? 1 : 0;
+    if (a.j0 < j1 && sh.nt - 1 - LAG - a.j0 >= 0) stage_images(a.ntb - 1 - LAG - a.j0);
     int cur = 0;
     __syncthreads();
     for (int j = a.j0; j < j1; j++) {
         const unsigned tag = a.tag0 + j;
-        const int g_img = a.ntb - 1 - j;
+        const int g_img = a.ntb - 1 - LAG - j;
+        const bool img = !REF || sh.nt - 2 - j >= 0;
         float *const UZ = S.halo[cur], *const pc = pO + cur * PT;
         // this step's residuals and scale: in flight until the increments are done
         float2 d = both(0.f);
-        const float scale = Cd::scaled ? b.scale[(long)B.s * b.nt_max + g_img] : 1.f;
+        const float scale = Cd::scaled && img ? b.scale[(long)B.s * b.nt_max + g_img] : 1.f;
         if (rec_rr >= 0 && rec_rr < nr) {
             const float *const res = b.rec + sh.rec_off + (long)(sh.nt - j - 1) * (sh.rx1 - sh.rx0) - sh.rx0 + ix;
             if (ix >= sh.rx0 && ix < sh.rx1) d.x = res[0];
             if (ix + 1 >= sh.rx0 && ix + 1 < sh.rx1) d.y = res[1];
         }
-        if (B.side) {
+        if (REF && B.side) {
+            // as the forward: psi_x, then zeta_x and what the side layers add to Dxx u_x
+            const float2 ax = ld2(S.ax + cx), bx = ld2(S.bx + cx);
+            for (int rr = 0; rr < nr; rr++) {
+                float *const ps = pS + rr * SD * WB;
+                put2(ps, keep(fma(bx, ld2(ps), mul(ax, scaled(ResWindow(pc + rr * OWN * PT).d1(), inv_dh))), nval));
+            }
+            res_side_sync(B);
+            for (int rr = 0; rr < nr; rr++) {
+                float *const ps = pS + rr * SD * WB;
+                const float2 gp = scaled(ResWindow(pc + rr * OWN * PT).d2(), inv_dh2), dx = ResWindow(ps).d1();
+                const float2 z = keep(res_zeta(true, bx, ld2(ps + WB), ax, gp, dx, inv_dh), nval);
+                const float2 t = res_term(true, dx, inv_dh, z);
+                const bool zl = B.iz0 + r0 + rr >= B.zb;
+                put2(ps + WB, z);
+                put2(ps + 2 * WB, make_float2(lay0 || zl ? t.x : 0.f, lay1 || (zl && nval > 1) ? t.y : 0.f));
+            }
+        }
+        if (!REF && B.side) {
             // Y_x of the side layers: Y' = -D(w) + b Y, w = u at layer points, 0 elsewhere; and a Y'
             const float2 ax = ld2(S.ax + cx), bx = ld2(S.bx + cx);
             for (int rr = 0; rr < nr; rr++) {
@@ -803,7 +830,31 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
         }
         if (j > a.j0 || load) res_halo_in<PT>(B, UZ, a.x, tag, &dead, b.status);
         __syncthreads();
-        if (B.bottom) {
+        if (REF && B.bottom) {
+            // psi_z, then zeta_z and what the bottom layer adds to Dzz u_z, as the forward
+            res_rows<PT>(B, bz0, bz1, UZ, [&](int r, const float2 *uz) {
+                float *const ps = S.zh + r * PT + ix;
+                put2(ps, keep(fma(both(S.bz[r]), ld2(ps), mul(both(S.az[r]), scaled(res_d1z(uz), inv_dh))), nval));
+                if (r >= 0 && r < nrow) put2(S.zo + (r * 2 + 1) * PT + ix, scaled(res_d2z(uz), inv_dh2));
+            });
+            __syncthreads();
+            res_rows<PT>(B, max(B.zb - 4 - B.iz0, 0), nrow, S.zh, [&](int r, const float2 *pz) {
+                float *const z = S.zo + r * 2 * PT + ix;
+                const float2 dz = res_d1z(pz);
+                float2 t;
+                if (B.iz0 + r >= B.zb) {
+                    const float2 n = keep(res_zeta(true, both(S.bz[r]), ld2(z), both(S.az[r]), ld2(z + PT), dz, inv_dh), nval);
+                    put2(z, n);
+                    t = res_term(true, dz, inv_dh, n);
+                } else {
+                    t = scaled(dz, inv_dh);
+                    t = make_float2(lay0 ? t.x : 0.f, lay1 ? t.y : 0.f);
+                }
+                put2(z + PT, t);
+            });
+            __syncthreads();
+        }
+        if (!REF && B.bottom) {
             // Y_z of the bottom layer's points of the own rows and 4 either side
             res_rows<PT>(B, bz0, bz1, UZ, [&](int r, const float2 *uz) {
                 const int iz = B.iz0 + r;
@@ -840,7 +891,7 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
                 win[rr + 8] = ld2(uc + (rr + 4) * PT);
                 float *const o = pO + rr * OWN * PT;
                 float2 ex = scaled(ResWindow(pc + rr * OWN * PT).d2(), inv_dh2), ez = scaled(res_d2z(win + rr), inv_dh2);
-                if (B.side) ex = add(ex, ld2(pS + (rr * SD + 4) * WB));
+                if (B.side) ex = add(ex, ld2(pS + (rr * SD + (REF ? 2 : 4)) * WB));
                 if (B.bottom) ez = add(ez, ld2(S.zo + ((r0 + rr) * 2 + 1) * PT + ix));
                 WP[rr] = add(WP[rr], ex);
                 WF[rr] = add(WF[rr], ez);
@@ -852,6 +903,7 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
                 LP[rr] = add(LP[rr], WP[rr]);
                 LF[rr] = add(LF[rr], WF[rr]);
                 make_u(rr, 1 - cur, LP[rr], LF[rr], true, tag + 1);
+                if (!img) continue;
                 const SI *const image = images + (long)(g_img - a.img_base) * 2 * b.slot + (long)rr * b.pitch;
                 const float2 gi = keep(mul(kk, Img::value(STAGE ? pI + rr * 2 * PT : image, inv_sc)), nval),
                              hi = keep(mul(kk, Img::value(STAGE ? pI + (rr * 2 + 1) * PT : image + b.slot, inv_sc)), nval);
@@ -860,7 +912,7 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
                 put2(o + 7 * PT, fma(gi, LF[rr], ld2(o + 7 * PT)));
             }
         }
-        if (j + 1 < j1) stage_images(g_img - 1);
+        if (j + 1 < j1 && (!REF || sh.nt - 3 - j >= 0)) stage_images(g_img - 1);
         __syncthreads();  // the next u; this one and Y read
         cur ^= 1;
     }
@@ -888,6 +940,58 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
             put2(b.cp[4] + i, ld2(S.zo + (r0 + rr) * 2 * PT + ix));
         }
     }
+}
+
+// ------------------------------------------------------------------ launches
+
+template <typename Args> using ResKernel = void (*)(Batch<float>, ResidentGrid, Args);
+
+template <int ST, bool REF> ResKernel<ResAdjArgs> res_adj_kernel(int pitch)
+{
+    switch (pitch) {
+    case 96: return k_resident_adj<ST, 96, REF>;
+    case 160: return k_resident_adj<ST, 160, REF>;
+    case 224: return k_resident_adj<ST, 224, REF>;
+    case 320: return k_resident_adj<ST, 320, REF>;
+    case 400: return k_resident_adj<ST, 400, REF>;
+    case 512: return k_resident_adj<ST, 512, REF>;
+    case 640: return k_resident_adj<ST, 640, REF>;
+    default: return nullptr;
+    }
+}
+template <bool REF> ResKernel<ResAdjArgs> res_adj_kernel(int store_type, int pitch)
+{
+    return store_type == kStoreHalf ? res_adj_kernel<kStoreHalf, REF>(pitch)
+           : store_type == kStoreBf16 ? res_adj_kernel<kStoreBf16, REF>(pitch) : res_adj_kernel<kStoreNative, REF>(pitch);
+}
+
+// Cooperative: every CTA of the launch is resident before any of them waits on another.
+template <typename Args>
+cudaError_t res_launch(ResKernel<Args> k, const Batch<float> &b, const ResidentSet &set, const Args &a, cudaStream_t st)
+{
+    if (!k) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(set.grid.n);
+    cfg.blockDim = dim3(set.threads);
+    cfg.dynamicSmemBytes = set.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, b, set.grid, a);
+}
+
+// Every kernel of a table may take `smem` bytes of dynamic shared memory.
+template <typename Kernel> bool res_allow(Kernel kernel, int smem)
+{
+    bool ok = true;
+    for (int st : {(int)kStoreNative, (int)kStoreHalf, (int)kStoreBf16})
+        for (int p : kResPitches)
+            if (const void *k = (const void *)kernel(st, p))
+                ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+    return ok;
 }
 
 }  // namespace fwi

@@ -2,7 +2,7 @@
 (environment FWI_CLUSTER=0), at the sizes where the row bands, column pairs and side layers are at
 their limits: odd and narrow windows, layers of 4 and 5 points, few rows, windows of several widths
 and lengths in one batch, several launches a batch, every image type, checkpoints and the
-reference mode (its forward).  The forward rounds as the passes do, the adjoint in another order.
+reference mode.  The forward rounds as the passes do, the adjoint in another order.
 Tolerances (relative L2), 2^-24 a step adding up over nt steps as a random walk, ten of it a step:
 10 x 2^-24 x sqrt(240) = 1e-5 for records and FP32-image gradients; with 16-bit images a last-bit
 difference may move an image by 2^-9 where it lies at a rounding boundary, a chance of 2^-7 at such a
@@ -25,6 +25,9 @@ CASES = [  # nx, nz, cpml, shots, store, images, mode, windows of several sizes
     (72, 56, 12, 34, "CHECKPOINT", "FP16", "EXACT", True),
     (209, 200, 20, 24, "FULL", "FP16", "EXACT", False),
     (149, 90, 12, 2, "FULL", "NATIVE", "REF_COMPAT", False),
+    (131, 77, 13, 4, "CHECKPOINT", "FP16", "REF_COMPAT", True),
+    (501, 60, 20, 1, "FULL", "BF16", "REF_COMPAT", False),
+    (53, 50, 5, 2, "CHECKPOINT", "NATIVE", "REF_COMPAT", False),
 ]
 
 
