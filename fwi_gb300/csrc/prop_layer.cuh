@@ -66,6 +66,15 @@ __device__ __forceinline__ void row12(const float *row, float *v)
     v[8] = a2.x; v[9] = a2.y; v[10] = a2.z; v[11] = a2.w;
 }
 
+// Whether the tile at (x0, z0) holds points of the side (bottom) layer or within 4 of it.  The terms of
+// the layer that it does not reach are zero: such tiles skip their loads and arithmetic (a uniform
+// branch; most tiles reach one kind only).
+__device__ __forceinline__ bool reaches_side(int x0, int nx, int cpml)
+{
+    return x0 < cpml + kRad || x0 + TT > nx - cpml - kRad;
+}
+__device__ __forceinline__ bool reaches_bottom(int z0, int nz, int cpml) { return z0 + TT > nz - cpml - kRad; }
+
 // ------------------------------------------------------------------ forward
 
 // Forward layer tiles (src/parallelcalls.cu:48-117 at the strip points):
@@ -92,6 +101,7 @@ k_fwd_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int g, int ntb
     const DevShot gsh = b.shots[blockIdx.z * sg];
     const int nx = gsh.nx, nz = b.nz, pitch = b.pitch, cpml = b.cpml;
     if (tile_role(x0, z0, nx, nz, cpml) != 2) return;
+    const bool hasx = reaches_side(x0, nx, cpml), hasz = reaches_bottom(z0, nz, cpml);
     const int na = active_shots(b, sg, act, false, g, ntb);
     if (na == 0) return;
     if (tid == 0) {
@@ -169,13 +179,13 @@ k_fwd_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int g, int ntb
         if (any) {  // own points: issued before the wait
             vP = ld4(Pv0 + so + ipt);
             vF = ld4(Fv0 + so + ipt);
-            if (anyS) {
+            if (anyS && hasx) {
                 zX = ld4(zx0 + so + ipt);
+                if (INLINE) pX = ld4(psx0 + so + ipt);
+            }
+            if (anyS && hasz) {
                 zZ = ld4(zz0 + so + ipt);
-                if (INLINE) {
-                    pX = ld4(psx0 + so + ipt);
-                    pZ = ld4(psz0 + so + ipt);
-                }
+                if (INLINE) pZ = ld4(psz0 + so + ipt);
             }
         }
         if (!stage_ready(&bar[a % kLayerStages], (a / kLayerStages) & 1, b.status)) {
@@ -186,20 +196,26 @@ k_fwd_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int g, int ntb
         float lmax = 0.f;
         if (INLINE) {
             // psi of the own band points (src/parallelcalls.cu:48-63); other cells stay 0
-            if (any && anyS) {
+            if (any && anyS && hasx) {
                 float pv[12];
                 row12(&S.P[r][c4], pv);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float px = 0.f;
+                    if (xl[q]) px = bx[q] * comp(pX, q) + ax[q] * (d1_row(pv, q) * b.inv_dh);
+                    S.SX[r][c4 + kRad + q] = px;
+                    if (xl[q]) psx0[so + ipt + q] = px;
+                }
+            }
+            if (any && anyS && hasz) {
                 float4 fz[9];
 #pragma unroll
                 for (int k = 0; k < 9; k++) fz[k] = ld4(&S.F[r + k][c4]);
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    float px = 0.f, pz = 0.f;
-                    if (xl[q]) px = bx[q] * comp(pX, q) + ax[q] * (d1_row(pv, q) * b.inv_dh);
+                    float pz = 0.f;
                     if (S4[q] && zl) pz = bz * comp(pZ, q) + az * (d1_col(fz, q) * b.inv_dh);
-                    S.SX[r][c4 + kRad + q] = px;
                     S.SZ[r + kRad][c4 + q] = pz;
-                    if (xl[q]) psx0[so + ipt + q] = px;
                     if (S4[q] && zl) psz0[so + ipt + q] = pz;
                 }
             }
@@ -219,27 +235,27 @@ k_fwd_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int g, int ntb
                 G[q] = gP[q];
                 H[q] = gF[q];
             }
-            if (anyS) {
+            if (anyS && hasx) {
                 float sx[12];
                 row12(&S.SX[r][c4], sx);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const float tx = d1_row(sx, q) * b.inv_dh;
+                    const float n = xl[q] ? bx[q] * comp(zX, q) + ax[q] * (gP[q] + tx) : 0.f;
+                    if (S4[q]) G[q] = gP[q] + (tx + n);
+                    if (xl[q]) zx0[so + ipt + q] = n;
+                }
+            }
+            if (anyS && hasz) {
                 float4 sz[9];
 #pragma unroll
                 for (int k = 0; k < 9; k++) sz[k] = ld4(&S.SZ[r + k][c4]);
-                float nzx[4], nzz[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const float tx = d1_row(sx, q) * b.inv_dh, tz = d1_col(sz, q) * b.inv_dh;
-                    nzx[q] = xl[q] ? bx[q] * comp(zX, q) + ax[q] * (gP[q] + tx) : 0.f;
-                    nzz[q] = (S4[q] && zl) ? bz * comp(zZ, q) + az * (gF[q] + tz) : 0.f;
-                    if (S4[q]) {
-                        G[q] = gP[q] + (tx + nzx[q]);
-                        H[q] = gF[q] + (tz + nzz[q]);
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    if (xl[q]) zx0[so + ipt + q] = nzx[q];
-                    if (S4[q] && zl) zz0[so + ipt + q] = nzz[q];
+                    const float tz = d1_col(sz, q) * b.inv_dh;
+                    const float n = (S4[q] && zl) ? bz * comp(zZ, q) + az * (gF[q] + tz) : 0.f;
+                    if (S4[q]) H[q] = gF[q] + (tz + n);
+                    if (S4[q] && zl) zz0[so + ipt + q] = n;
                 }
             }
             const float w = sh.w;
@@ -364,6 +380,7 @@ k_adj_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int j, int ntb
     const int nx = gsh.nx, nz = b.nz, pitch = b.pitch, cpml = b.cpml;
     const int aw = EXACT ? cpml + kRad : cpml;
     if (tile_role(x0, z0, nx, nz, aw) != 2) return;
+    const bool hasx = reaches_side(x0, nx, cpml), hasz = reaches_bottom(z0, nz, cpml);
     const int na = active_shots(b, sg, act, true, j, ntb);
     if (na == 0) return;
     const int lag = EXACT ? 0 : 1;
@@ -499,7 +516,8 @@ k_adj_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int j, int ntb
             if (!EXACT && anyS)
                 for (int k = 0; k < 4; k++) zt[k] = ld4(b.cp[4 + k] + so + ipt);
             if (INLINE && anyS)  // EXACT: Yx, Yz; reference: the four psi (updated in place)
-                for (int k = 0; k < (EXACT ? 2 : 4); k++) yo[k] = ld4(b.cp[k] + so + ipt);
+                for (int k = 0; k < (EXACT ? 2 : 4); k++)
+                    if (!EXACT || (k == 0 ? hasx : hasz)) yo[k] = ld4(b.cp[k] + so + ipt);
         }
         if (!stage_ready(&bar[a % kLayerStages], (a / kLayerStages) & 1, b.status)) {
             drain_stages_n(bar, a, na, kLayerStages);
@@ -534,15 +552,20 @@ k_adj_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int j, int ntb
                     const float axq = axw[4 + q], bxq_ = bxq[q], az = azw[4], bz = bzr;
                     const long i = so + ipt + q;
                     if (EXACT) {
-                        const float gq = U[r][c + kRad], hq = V[r + kRad][c];
-                        const float zxo = S.A[r][c + kRad], zzo = S.C[r + kRad][c];
-                        WX[r][c + kRad] = S4[q] ? gq + axq * (gq + bxq_ * zxo) : 0.f;
-                        WZ[r + kRad][c] = S4[q] ? hq + az * (hq + bz * zzo) : 0.f;
-                        const float zxn = xl ? gq + bxq_ * zxo : 0.f, zzn = zl ? hq + bz * zzo : 0.f;
-                        S.A[r][c + kRad] = zxn;  // own cell: Z' replaces the old Z
-                        S.C[r + kRad][c] = zzn;
-                        if (xl) b.cp[3 - zsel][i] = zxn;
-                        if (zl) b.cp[5 - zsel][i] = zzn;
+                        if (hasx) {
+                            const float gq = U[r][c + kRad], zxo = S.A[r][c + kRad];
+                            WX[r][c + kRad] = S4[q] ? gq + axq * (gq + bxq_ * zxo) : 0.f;
+                            const float zxn = xl ? gq + bxq_ * zxo : 0.f;
+                            S.A[r][c + kRad] = zxn;  // own cell: Z' replaces the old Z
+                            if (xl) b.cp[3 - zsel][i] = zxn;
+                        }
+                        if (hasz) {
+                            const float hq = V[r + kRad][c], zzo = S.C[r + kRad][c];
+                            WZ[r + kRad][c] = S4[q] ? hq + az * (hq + bz * zzo) : 0.f;
+                            const float zzn = zl ? hq + bz * zzo : 0.f;
+                            S.C[r + kRad][c] = zzn;
+                            if (zl) b.cp[5 - zsel][i] = zzn;
+                        }
                     } else {
                         float d1 = 0.f, d3 = 0.f, d2 = 0.f, d4 = 0.f;
 #pragma unroll
@@ -584,19 +607,23 @@ k_adj_layer(Batch<float> b, const __grid_constant__ TmaMaps maps, int j, int ntb
                         const int ix = ix0 + q, c = c4 + q;
                         const bool xl = S4[q] && (ix < cpml || ix > nx - cpml - 1);
                         const bool zl = S4[q] && iz > nz - cpml - 1;
-                        float ax_ = 0.f, az_ = 0.f;
-#pragma unroll
-                        for (int k = 1; k <= 4; k++) {
-                            ax_ += c1[k - 1] * (WX[r][c + kRad + k] - WX[r][c + kRad - k]);
-                            az_ += c1[k - 1] * (WZ[r + kRad + k][c] - WZ[r + kRad - k][c]);
-                        }
-                        const float yx = xl ? -ax_ * b.inv_dh + bxq[q] * comp(yo[0], q) : 0.f;
-                        const float yz = zl ? -az_ * b.inv_dh + bzr * comp(yo[1], q) : 0.f;
-                        S.B[r][c + kRad] = yx;
-                        S.D[r + kRad][c] = yz;
                         const long i = so + ipt + q;
-                        if (xl) b.cp[0][i] = yx;
-                        if (zl) b.cp[1][i] = yz;
+                        if (hasx) {
+                            float ax_ = 0.f;
+#pragma unroll
+                            for (int k = 1; k <= 4; k++) ax_ += c1[k - 1] * (WX[r][c + kRad + k] - WX[r][c + kRad - k]);
+                            const float yx = xl ? -ax_ * b.inv_dh + bxq[q] * comp(yo[0], q) : 0.f;
+                            S.B[r][c + kRad] = yx;
+                            if (xl) b.cp[0][i] = yx;
+                        }
+                        if (hasz) {
+                            float az_ = 0.f;
+#pragma unroll
+                            for (int k = 1; k <= 4; k++) az_ += c1[k - 1] * (WZ[r + kRad + k][c] - WZ[r + kRad - k][c]);
+                            const float yz = zl ? -az_ * b.inv_dh + bzr * comp(yo[1], q) : 0.f;
+                            S.D[r + kRad][c] = yz;
+                            if (zl) b.cp[1][i] = yz;
+                        }
                     }
                 }
                 __syncthreads();
