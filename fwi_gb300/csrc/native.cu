@@ -1134,13 +1134,6 @@ template <typename T> struct Ctx : CtxBase {
         return FWI_OK;
     }
 
-    // Shots per group of the interior tile passes (a group of several windows
-    // runs their MIXED kernels; the layer passes then take one shot per
-    // block).  The tile passes are latency-bound, so many short blocks beat
-    // few long ones: the
-    // group count gives about three waves of adjoint tile blocks (3 resident
-    // per SM).  Measured on 601 x 301, 32 shots: 5 shots
-    // per group (7 groups) 56.8 shots/s, 8: 53.8, 3: 52.3, 16: 40.6.
     static bool uniform_windows(const std::vector<DevShot> &bs)
     {
         for (const DevShot &d : bs)
@@ -1148,7 +1141,17 @@ template <typename T> struct Ctx : CtxBase {
         return true;
     }
 
-    int shots_per_group(const std::vector<DevShot> &bs, int nxm) const
+    // Shots per group of the interior tile passes (a group of several windows
+    // runs their MIXED kernels; the layer passes then take one shot per
+    // block).  A block pays for its start (the list of shots, the adjoint's model
+    // tiles and gradient sums) once a group; blocks too few or too long leave the last
+    // wave empty.  Forward: 9 blocks an SM (4 resident), adjoint 4 (3 resident).  Adjoint
+    // microseconds a step with 9 -> 4 blocks an SM (with the recompute of checkpoint storage, the
+    // rebuild of boundary storage): 32 of 609 x 309 98.8 -> 96.0, 7 of 700 x 250 33.7 -> 28.5, 3 of
+    // 900 x 600 44.8 -> 35.1, 5 of 800 x 300 (boundary) 37.1 -> 29.2, 24 of 700 x 300 (boundary) 95.3 ->
+    // 93.6 (2 blocks: 107).  Forward with 9 / 7 / 12 blocks: 32 of 609 x 309 48.4 / 50.9 / 49.5, 40 of
+    // 420 x 200 30.8 / 32.8 / 31.6, 24 of 700 x 300 41.7 / 42.2 / 44.0.
+    int shots_per_group(const std::vector<DevShot> &bs, int nxm, bool adjoint) const
     {
         if (!use_tma) return 1;
         if (const char *e = getenv("FWI_SHOTS_PER_GROUP")) {  // tuning override
@@ -1156,20 +1159,22 @@ template <typename T> struct Ctx : CtxBase {
             if (v >= 1) return std::min(v, 64);
         }
         const long tiles = (long)((nxm - 5) / 32 + 1) * ((nz - 5) / 32 + 1);  // tiles holding interior points
-        const long slots = 3L * n_sm;
+        const long blocks = (adjoint ? 4L : 9L) * n_sm;
         const long nb = (long)bs.size();
-        const long groups = std::max(1L, std::min(nb, (3 * slots + tiles / 2) / tiles));
+        const long groups = std::max(1L, std::min(nb, (blocks + tiles / 2) / tiles));
         const long sg = (nb + groups - 1) / groups;
         return (int)std::max(1L, std::min(sg, 64L));
     }
 
-    // Shots per group of the layer tiles (with identical windows).  They run
-    // on the side stream beside the interior tiles; the group count gives
-    // about half a wave of adjoint blocks (3 per SM): short enough a
-    // pass, without a block prologue per shot.  Measured on 601 x 301, 32
-    // shots (54 layer tiles): 8 shots per group 60.2 shots/s, 5: 59.1,
-    // 16: 54.9, 2: 56.6, 1: 53.4.
-    int layer_shots_per_group(int nb, int nxm, int xbase, int zbase) const
+    // Shots per group of the layer tiles (with identical windows).  They run on
+    // the side stream beside the interior tiles, in blocks that take half an SM's
+    // registers (the adjoint's also half its shared memory): forward about 7/3 blocks an SM, adjoint
+    // 3/4 (its blocks start dear, and an SM with two of them has no room for interior tiles).
+    // Microseconds a forward / adjoint step, 3/2 blocks an SM for both -> this: 32 of 609 x 309
+    // 50.7 / 101.6 -> 48.4 / 98.7 (adjoint with 1/2: 100.0, 1: 100.9), 16 forward 25.2 -> 24.0, 4 of
+    // 2009 x 809 adjoint 112.3 -> 108.4, 4 of 1009 x 409 (full storage) 33.6 -> 29.1, 40 of 420 x 200
+    // 32.8 / 69.4 -> 30.8 / 68.1 (1/2: 72.1).
+    int layer_shots_per_group(int nb, int nxm, int xbase, int zbase, bool adjoint) const
     {
         if (const char *e = getenv("FWI_LAYER_SHOTS_PER_GROUP")) {  // tuning override
             const int v = atoi(e);
@@ -1179,7 +1184,7 @@ template <typename T> struct Ctx : CtxBase {
         for (int z0 = zbase; z0 < nz; z0 += fwi::kTileEdge)
             for (int x0 = xbase; x0 < nxm; x0 += fwi::kTileEdge)
                 tiles += fwi::tile_role(x0, z0, nxm, nz, cfg.cpml + fwi::kRad) == 2;
-        const long slots = 3L * n_sm / 2;
+        const long slots = adjoint ? 3L * n_sm / 4 : 7L * n_sm / 3;
         const long groups = std::max(1L, std::min((long)nb, (slots + tiles / 2) / std::max(1L, tiles)));
         return (int)std::max(1L, std::min((nb + groups - 1) / groups, 64L));
     }
@@ -1224,15 +1229,15 @@ template <typename T> struct Ctx : CtxBase {
         return {(long)bs.size(), (long)nxm, uniform_windows(bs) ? 1L : 0L, (long)cfg.mode, (long)store_type()};
     }
 
-    Choice default_choice(const std::vector<DevShot> &bs, int nxm) const
+    Choice default_choice(const std::vector<DevShot> &bs, int nxm, bool adjoint) const
     {
         Choice c;
-        c.sg = shots_per_group(bs, nxm);
+        c.sg = shots_per_group(bs, nxm, adjoint);
         fwi::TileGrid tg;
         if (use_tma && uniform_windows(bs)) tg = fwi::tile_grid(nxm, nz, cfg.cpml);
         c.inline_strip = tg.inline_strip ? 1 : 0;
-        c.sg_layer = c.sg == 1 || !uniform_windows(bs) ? 1
-                                                       : layer_shots_per_group((int)bs.size(), nxm, tg.xbase, tg.zbase);
+        c.sg_layer =
+            use_tma && uniform_windows(bs) ? layer_shots_per_group((int)bs.size(), nxm, tg.xbase, tg.zbase, adjoint) : 1;
         return c;
     }
 
@@ -1241,8 +1246,7 @@ template <typename T> struct Ctx : CtxBase {
         const std::vector<long> key = choice_key(bs, nxm);
         for (const Tuned &t : tuned)
             if (t.key == key) return t.c;
-        const Choice d = default_choice(bs, nxm);
-        return {d, d};
+        return {default_choice(bs, nxm, false), default_choice(bs, nxm, true)};
     }
 
     void record_choice(const std::vector<long> &key, const Choices &c)
@@ -2270,8 +2274,7 @@ template <typename T> struct Ctx : CtxBase {
             TRY(cudaMemcpyAsync(shots, bs.data(), nb * sizeof(DevShot), cudaMemcpyHostToDevice, st));
             const int K = std::min(steps, ntb);
             const size_t lb = (size_t)nb * slot * sizeof(T);
-            const Choice dflt = default_choice(bs, nxm);
-            Choices best{dflt, dflt};
+            Choices best{default_choice(bs, nxm, false), default_choice(bs, nxm, true)};
             // device time per step of phase ph (0 forward, 1 adjoint) with choice c.  The adjoint
             // steps run beside what runs beside them in a gradient call: with checkpoint storage
             // the segment recompute (forward steps on the recompute streams, with the forward's
@@ -2349,8 +2352,8 @@ template <typename T> struct Ctx : CtxBase {
             double t_best[2] = {0, 0}, t_dflt[2] = {0, 0}, t = 0;
             int trials = 0;
             for (int ph = 0; ph < 2; ph++) {
-                if ((rc = trial(dflt, ph, t))) return rc;  // warm-up
-                if ((rc = timed(dflt, ph, t_dflt[ph]))) return rc;
+                if ((rc = trial(ph == 0 ? best.fwd : best.adj, ph, t))) return rc;  // warm-up
+                if ((rc = timed(ph == 0 ? best.fwd : best.adj, ph, t_dflt[ph]))) return rc;
                 t_best[ph] = t_dflt[ph];
                 trials++;
                 Choice &bp = ph == 0 ? best.fwd : best.adj;
