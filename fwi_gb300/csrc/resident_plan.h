@@ -26,7 +26,11 @@ constexpr int kResMaxCpml = 32;   // the widest layer whose side columns fit one
 constexpr int kResFwdOwn = 5, kResAdjOwn = 8;    // own-row arrays
 constexpr int kResFwdSide = 3, kResAdjSide = 5;  // side arrays
 // Shared row pitches the kernels are compiled for, and at each the threads of a CTA at most (the
-// fewer, the more registers each) and the rows a thread holds at most.
+// fewer, the more registers each) and the rows a thread holds at most (the more, the fewer launches a
+// batch takes; past these they spill).  Microseconds a forward / adjoint step, to 320 columns with 512
+// threads x 4 rows -> 448 x 5 / 4: one 209 x 209 3.15 / 3.50 -> 3.05 / 3.48, 8 of them 4.9 / 4.6 -> 4.8 / 4.6,
+// 16 of 300 x 300 18.0 / 36.0 -> 14.1 / 33.3 (448 x 6: 11.5 / 30.2, but one 209 x 209 3.22); beyond with
+// 640 x 6 forward -> 640 x 4: 8 of 400 x 200 8.7 -> 7.4.
 constexpr int kResPitches[] = {96, 160, 224, 320, 400, 512, 640};
 constexpr int kResFwdPitch = 400;  // the widest forward kernel's
 struct ResShape {
@@ -34,7 +38,7 @@ struct ResShape {
 };
 __host__ __device__ constexpr ResShape res_shape(int pitch)
 {
-    return pitch <= 320 ? ResShape{512, 4, 4} : ResShape{640, 6, 4};
+    return pitch <= 320 ? ResShape{448, 5, 4} : ResShape{640, 4, 4};
 }
 
 // The pitch for windows nx wide (rows end at a multiple of 4), 0: none.
