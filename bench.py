@@ -458,8 +458,8 @@ def native_arm(args, rank, world, dist):
 
 def single_shot_c1(args, fwi_gb300, torch, dev, steps=10, warmup=3):
     """The plain single-shot gradient (C1: 209 x 209, nt 2000, one shot, full image storage) on the
-    small-shot cluster path (one 16-CTA cluster takes the shot through every step in one launch per
-    phase) and, beside it, on the per-step tile passes (FWI_CLUSTER=0); device-resident inputs,
+    on-chip path (key "cluster": one launch takes the shot through every step of a phase, resident over
+    the whole GPU) and, beside it, on the per-step tile passes (FWI_CLUSTER=0); device-resident inputs,
     CUDA events over `steps` gradients after `warmup`."""
     from fwi_gb300 import synth
     w = synth.WORKLOADS["C1"]()
@@ -503,7 +503,7 @@ def single_shot_c1(args, fwi_gb300, torch, dev, steps=10, warmup=3):
         del c
     os.environ.pop("FWI_CLUSTER", None)
     out["cluster_speedup_over_tile_passes"] = round(out["cluster"]["value"] / out["tile_passes"]["value"], 3)
-    # the same small shots in a batch: one cluster per shot, the clusters side by side on the GPU
+    # the same shots in a batch, side by side on the GPU
     nb = 8
     base = w.shots[0]
     many = [dict(base, sx=int(8 + (w.nx - 16) * (k + 0.5) / nb)) for k in range(nb)]
