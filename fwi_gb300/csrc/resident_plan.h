@@ -320,6 +320,10 @@ inline bool resident_plan(const std::vector<int> &nx, int nz, int cpml, size_t s
             }
         }
         g.n = c;
+        if (set.smem > smem_limit) {  // a grid lower than the bottom layer: not a window the library takes
+            out.clear();
+            return false;
+        }
         out.push_back(set);
         s0 = s1;
     }
