@@ -27,13 +27,15 @@ using fwi::Coef;
 using fwi::in_strip;
 using fwi::interior;
 using fwi::StripMap;
+using fwi::widen;
 
 // A block's outputs, one a thread.  What bounds the passes is the FP64 pipe (64 cycles a warp
 // instruction on an SM quarter): small tiles spread a small grid over all of it, and the fewest
 // FP64 operations a point count (RefDiv below).  One shot of the reference's sequence, 209 x 209, 300
 // steps each way: 59.7 ms with 32 x 32 tiles of 4 points a thread, 32.2 with 16 x 8, 29.1 without
-// the separate entryPoint pass and with strip blocks of 64 threads, 21.7 with the division below;
-// 609 x 309, 100 steps: 29.2, 20.8, 20.0, 13.7.  (FP32 to FP64 by integer operations measured no faster.)
+// the separate entryPoint pass and with strip blocks of 64 threads, 21.7 with the division below,
+// 20.0 with FP32 widened by integer operations (common.cuh); 609 x 309, 100 steps: 29.2, 20.8, 20.0,
+// 13.5, 11.8.
 constexpr int TX = 16, TZ = 8;
 constexpr int XW = TX + 2 * fwi::kRad, ZH = TZ + 2 * fwi::kRad;
 
@@ -75,15 +77,15 @@ __device__ __forceinline__ double ref_div(double s, const RefDiv &v)
 
 template <typename V> __device__ __forceinline__ double ref_first(V v, const RefDiv &dh)
 {
-    return ref_div((4 / 5.) * (v(1) - v(-1)) - (1 / 5.) * (v(2) - v(-2)) + (4 / 105.) * (v(3) - v(-3)) -
-                   (1 / 280.) * (v(4) - v(-4)),
+    return ref_div((4 / 5.) * widen(v(1) - v(-1)) - (1 / 5.) * widen(v(2) - v(-2)) + (4 / 105.) * widen(v(3) - v(-3)) -
+                   (1 / 280.) * widen(v(4) - v(-4)),
                    dh);
 }
 
 template <typename V> __device__ __forceinline__ double ref_second(V v, const RefDiv &dh2)
 {
-    return ref_div(-(205 / 72.) * v(0) + (8 / 5.) * (v(1) + v(-1)) - (1 / 5.) * (v(2) + v(-2)) +
-                   (8 / 315.) * (v(3) + v(-3)) - (1 / 560.) * (v(4) + v(-4)),
+    return ref_div(-(205 / 72.) * widen(v(0)) + (8 / 5.) * widen(v(1) + v(-1)) - (1 / 5.) * widen(v(2) + v(-2)) +
+                   (8 / 315.) * widen(v(3) + v(-3)) - (1 / 560.) * widen(v(4) + v(-4)),
                    dh2);
 }
 

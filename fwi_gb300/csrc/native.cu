@@ -321,21 +321,10 @@ template <typename T> struct alignas(16) Pack {
 // operations, x + k u is rounded from error-free FP32 parts, no FP64 operation by 1 or 0; copies made by
 // the pass that has the values, scalar steps by the last block of the reduction that feeds them.
 // First step and 5 directions and updates on 2009 x 809: 4.90 ms before, 3.37 with FP64
-// conversions in 2 blocks an SM, 1.9 now.
+// conversions in 2 blocks an SM, 1.8 now.
 
-// The rare cases, out of line: as branches the compiler would run their FP64 operations for every value.
-__device__ __noinline__ double widen_any(float v) { return (double)v; }
+// The rare case, out of line: as a branch the compiler would run its FP64 operations for every value.
 __device__ __noinline__ float axpy_any(float x, float u, double k) { return (float)((double)x + k * (double)u); }
-
-__device__ __forceinline__ double widen(double v) { return v; }
-// Exact; all but normal values and zeros (rare) by the conversion.
-__device__ __forceinline__ double widen(float v)
-{
-    const unsigned u = __float_as_uint(v), e = u & 0x7f800000u;
-    if (e == 0x7f800000u || (e == 0 && (u << 1) != 0)) return widen_any(v);
-    const unsigned hi = (u & 0x80000000u) | (e ? ((u & 0x7fffffffu) >> 3) + 0x38000000u : 0u);
-    return __hiloint2double((int)hi, (int)(u << 29));
-}
 
 // An FP64 coefficient, for FP32 operands in two parts (48 bits) when it lies well inside FP32's range.
 template <typename T> struct LbCoef {
@@ -435,10 +424,10 @@ __global__ void __launch_bounds__(kRedThreads) k_lb_pair(Tri<T> s, Tri<T> y, CTr
             for (int q = 0; q < P::N; q++) {
                 sv.v[q] = mv.v[q] - mo.v[q];
                 yv.v[q] = gv.v[q] - go.v[q];
-                const double sd = widen(sv.v[q]), yd = widen(yv.v[q]);
+                const double sd = fwi::widen(sv.v[q]), yd = fwi::widen(yv.v[q]);
                 v[0][p] += yd * sd;
                 v[1][p] += yd * yd;
-                v[2][p] += sd * widen(gv.v[q]);
+                v[2][p] += sd * fwi::widen(gv.v[q]);
                 v[3][p] += sd * sd;
             }
             sv.put(s.p[p] + i);
@@ -464,7 +453,7 @@ __global__ void __launch_bounds__(kRedThreads) k_lb_first(CTri<T> m, Tri<T> mb, 
             gv.put(gb.p[p] + i);
 #pragma unroll
             for (int q = 0; q < P::N; q++) {
-                const double w = widen(gv.v[q]);
+                const double w = fwi::widen(gv.v[q]);
                 v[0][p] += w * w;
             }
         }
@@ -496,7 +485,7 @@ __global__ void __launch_bounds__(kRedThreads) k_lb_axpy_dot(Tri<T> x, CTri<T> s
             for (int q = 0; q < P::N; q++) {
                 xv.v[q] = k1[p].axpy(xv.v[q], uv.v[q]);
                 if (GAMMA) xv.v[q] = gam[p].scale(xv.v[q]);
-                if (AFTER != LB_LAST) v[0][p] += widen(nv.v[q]) * widen(xv.v[q]);
+                if (AFTER != LB_LAST) v[0][p] += fwi::widen(nv.v[q]) * fwi::widen(xv.v[q]);
             }
             xv.put(x.p[p] + i);
         }
