@@ -18,6 +18,7 @@
 #include "../../include/fwi_compat.h"
 #include "common.cuh"
 #include "tile.cuh"
+#include "widen.cuh"
 
 #include <cmath>
 
@@ -34,7 +35,7 @@ using fwi::widen;
 // FP64 operations a point count (RefDiv below).  One shot of the reference's sequence, 209 x 209, 300
 // steps each way: 59.7 ms with 32 x 32 tiles of 4 points a thread, 32.2 with 16 x 8, 29.1 without
 // the separate entryPoint pass and with strip blocks of 64 threads, 21.7 with the division below,
-// 20.0 with FP32 widened by integer operations (common.cuh); 609 x 309, 100 steps: 29.2, 20.8, 20.0,
+// 20.0 with FP32 widened by integer operations (widen.cuh); 609 x 309, 100 steps: 29.2, 20.8, 20.0,
 // 13.5, 11.8.
 constexpr int TX = 16, TZ = 8;
 constexpr int XW = TX + 2 * fwi::kRad, ZH = TZ + 2 * fwi::kRad;

@@ -15,6 +15,7 @@
 #include "prop.h"
 #include "resident_plan.h"
 #include "tma.cuh"
+#include "widen.cuh"
 
 #include <cuda_fp16.h>
 #include <nvtx3/nvToolsExt.h>
@@ -623,7 +624,7 @@ struct CtxBase {
     int last_cuda = 0;
     int n_sm = 1;        // streaming multiprocessors of the context's device
     int red_blocks = 2;  // blocks of the reduction kernels: 2 per SM
-    int lb_blocks = 3;   // of the L-BFGS passes: 3 per SM (5 pairs, 2009 x 809: 391 us; 2: 432, 4: 412, 8: 546)
+    int lb_blocks = 3;   // of the L-BFGS passes: 3 per SM (5 pairs, 2009 x 809: 391 us; 2: 432, 4: 412, 8: 546, before values widened as now)
     unsigned eg(long n) const { return elt_grid(n, n_sm); }
     float timing[4] = {0, 0, 0, 0};
     long launches = 0;
