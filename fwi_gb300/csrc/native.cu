@@ -1337,7 +1337,7 @@ template <typename T> struct Ctx : CtxBase {
     //    3.0 -> 2.5, 12 of 400 x 400 (1.9 M points) 4.5 -> 4.3, 16 (2.6 M) 8.3 -> 8.9 (300 steps); one
     //    500 x 200 1.7 -> 2.3 (300 steps): wide windows leave a CTA few rows and long halos.
     //  - Adjoint of stored images: windows to 400 wide; to 640 where all shots run at once.  Tiles ->
-    //    resident: 40 of 320 x 300 11.9 -> 8.1 (200 steps), one 609 x 309 3.4 -> 2.5, three (two
+    //    resident: 40 of 320 x 300 11.9 -> 8.1 (200 steps), one 609 x 309 3.4 -> 2.0, three (two
     //    launches) 6.0 -> 6.4 (300 and 400 steps).
     bool resident_path(const std::vector<DevShot> &bs, int nxm, bool want_grad, ResidentRun &run)
     {

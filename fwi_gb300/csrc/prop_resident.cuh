@@ -16,7 +16,7 @@
 // 16-bit images travels the same way (one 8-byte word per CTA).  Words of step t go to copy t mod
 // kResSlots.  No copy is overwritten unread: a CTA that writes step t + 1 has its neighbours' rows
 // of step t, so they have read theirs of step t - 1, the next ones theirs of step t - 2, and CTAs
-// three apart (the farthest that exchange rows: bands have at least 3) theirs of step t - 3.
+// kResReach apart (the farthest that exchange rows) theirs of step t - kResReach.
 // Every wait is bounded; one that gives up sets the status word, and its CTA waits no more.
 //
 // A thread owns 2 columns x R consecutive rows; the z-window of its rows slides through registers.
@@ -30,16 +30,16 @@
 // residual, next u and Z, edge rows out, imaging.  A block barrier ends each part.  Arithmetic on
 // pairs of columns (FADD2, FFMA2) halves the instructions of the stencils.
 //
-// What bounds it: latency.  A C1 step (209 x 209, 67 bands of 3 rows) is 1.9 us of forward (2.3 us
-// of adjoint) arithmetic between block barriers, about 4.5 cycles an instruction of the longest
+// What bounds it: latency.  A C1 step (209 x 209, 100 bands of 2 rows; 2.8 us forward, 3.3 us adjoint) is 1.8 us (2.2 us
+// of adjoint) of arithmetic between block barriers, about 4.5 cycles an instruction of the longest
 // thread, and 1.0 us for the exchange (a bare exchange of one row measures 0.9 - 1.1 us a step, of
 // 4 rows of 100 pairs 1.3 us, whatever the number of CTAs; flags with fences 1.7 - 2.0 us).  So: the
 // fewest barriers (two levels, one barrier a part), values published from the registers that hold
 // them, registers over shared memory up to the point where they spill (spills miss the small L1
 // that this much shared memory leaves), 2 columns a thread (4: C1 3.75 us an adjoint step against
 // 3.3, fewer threads a band).  A 2000-step C1 gradient with FP32 images took 16.8 ms on one 16-CTA
-// cluster, takes 13.0; 8 shots with FP16 images 36.2 -> 18.9 (two waves of clusters before); the
-// adjoint of one 609 x 309 shot 34 -> 26 ms for 3000 steps.
+// cluster, takes 12.3; 8 shots with FP16 images 36.2 -> 18.6 (two waves of clusters before); the
+// adjoint of one 609 x 309 shot 34 -> 20 ms for 3000 steps.
 #pragma once
 
 #include "prop_layer.cuh"
@@ -269,7 +269,7 @@ struct ResBand {
         use = seg < nlane && (side ? p.nside > 0 : p.nq > p.nside);
         // rows the CTAs above (below) read as their lower (upper) halo
         int lo = 0, hi = 0;
-        for (int c = max(k0, self - 3); c < min(k1, self + 4); c++) {
+        for (int c = max(k0, self - kResReach); c <= min(k1 - 1, self + kResReach); c++) {
             if (c == self) continue;
             const int a = grid.row0[c], e = a + grid.nrow[c], h = res_halo(a, e, nz, cpml);
             if (c < self) lo = max(lo, e + h - row0);

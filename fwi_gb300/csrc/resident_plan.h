@@ -19,8 +19,11 @@
 namespace fwi {
 
 constexpr int kResMaxCtas = 160;  // CTAs of a launch (one per SM)
-constexpr int kResMinRows = 3;    // rows of a CTA at least: its halo then comes from three neighbours either side
-constexpr int kResSlots = 4;      // copies of the exchanged rows (step modulo kResSlots)
+constexpr int kResMinRows = 2;    // rows of a CTA at least (3: one C1 3.03 / 3.47 us a step against 2.84 / 3.27, the adjoint of one
+                                  // 609 x 309 8.5 against 6.7; 1: C1 2.75 / 3.20, but 4 of 300 x 200 5.1 / 4.7 against 4.5 / 4.0)
+constexpr int kResReach = (2 * kRad + kResMinRows - 1) / kResMinRows;  // its halo comes from so many CTAs either side
+constexpr int kResSlots = 8;      // copies of the exchanged rows (step modulo kResSlots): more than kResReach
+static_assert(kResSlots > kResReach && (kResSlots & (kResSlots - 1)) == 0, "copies of the exchanged rows");
 constexpr int kResSide = 96;      // floats of a side array's row
 constexpr int kResMaxCpml = 32;   // the widest layer whose side columns fit one
 constexpr int kResFwdOwn = 5, kResAdjOwn = 8;    // own-row arrays

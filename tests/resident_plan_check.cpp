@@ -1,7 +1,7 @@
 // Checks the resident path's plan (fwi_gb300/csrc/resident_plan.h) over a sweep of windows, grid
 // heights, layer widths and batches: every launch within the SMs, threads, registers and shared
 // memory; rows covered once; every index the kernels form inside its array; every halo row a CTA
-// reads published by an owner at most three CTAs away, and no copy of an exchanged row overwritten
+// reads published by an owner at most kResReach CTAs away, and no copy of an exchanged row overwritten
 // before its readers are done (the most steps such CTAs can be apart).
 #include <cstdio>
 #include <cstdlib>
@@ -64,16 +64,16 @@ static bool check_cta(const ResidentSet &set, int c, int nx, int nz, int cpml, i
         CHECK((col < cpml || col > nx - cpml - 1) && col >= 4 && col < nx - 4);
         CHECK(G.col(col) >= 0 && G.col(col) < kResSide && col + 4 < pt);
     }
-    // halo rows: published by their owner, at most three CTAs away, and the window rows inside
+    // halo rows: published by their owner, at most kResReach CTAs away, and the window rows inside
     for (int h = 0; h < 2 * hr; h++) {
         const int r = h < hr ? h - hr : nrow + h - hr, gi = row0 + r;
         if (gi < 0 || gi >= nzi) continue;
         int owner = -1;
         for (int k = g.first[c]; k < g.first[c] + g.count[c]; k++)
             if (gi >= g.row0[k] && gi < g.row0[k] + g.nrow[k]) owner = k;
-        CHECK(owner >= 0 && owner != c && std::abs(owner - c) <= 3);
+        CHECK(owner >= 0 && owner != c && std::abs(owner - c) <= kResReach);
         int lo = 0, hi = 0;
-        for (int k = std::max((int)g.first[c], owner - 3); k < std::min(g.first[c] + g.count[c], owner + 4); k++) {
+        for (int k = std::max((int)g.first[c], owner - kResReach); k < std::min(g.first[c] + g.count[c], owner + kResReach + 1); k++) {
             if (k == owner) continue;
             const int a = g.row0[k], e = a + g.nrow[k], hk = res_halo(a, e, nz, cpml);
             if (k < owner) lo = std::max(lo, e + hk - g.row0[owner]);
