@@ -19,10 +19,14 @@
 namespace fwi {
 
 constexpr int kResMaxCtas = 160;  // CTAs of a launch (one per SM)
-constexpr int kResMinRows = 2;    // rows of a CTA at least (3: one C1 3.03 / 3.47 us a step against 2.84 / 3.27, the adjoint of one
-                                  // 609 x 309 8.5 against 6.7; 1: C1 2.75 / 3.20, but 4 of 300 x 200 5.1 / 4.7 against 4.5 / 4.0)
-constexpr int kResReach = (2 * kRad + kResMinRows - 1) / kResMinRows;  // its halo comes from so many CTAs either side
-constexpr int kResSlots = 8;      // copies of the exchanged rows (step modulo kResSlots): more than kResReach
+// Rows of a CTA at least: 1 for a shot that has the GPU to itself, 2 beside others, which leave it
+// fewer CTAs, better spent on shorter upper bands.  Microseconds a forward / adjoint step with 3, 2, 1:
+// one C1 shot 3.03 / 3.47, 2.84 / 3.27, 2.75 / 3.20, one 400 x 200 5.2 / 4.9, 5.0 / 4.4, 4.8 / 3.9, the adjoint
+// of one 609 x 309 8.5, 6.7, 6.6; 4 shots of 300 x 200 4.6 / 4.0, 4.5 / 4.0, 5.0 / 4.7.
+constexpr int kResMinRows = 1;
+inline int res_min_rows(int nshots) { return nshots == 1 ? kResMinRows : 2; }
+constexpr int kResReach = (2 * kRad + kResMinRows - 1) / kResMinRows;  // a halo comes from so many CTAs either side at most
+constexpr int kResSlots = 16;     // copies of the exchanged rows (step modulo kResSlots): more than kResReach
 static_assert(kResSlots > kResReach && (kResSlots & (kResSlots - 1)) == 0, "copies of the exchanged rows");
 constexpr int kResSide = 96;      // floats of a side array's row
 constexpr int kResMaxCpml = 32;   // the widest layer whose side columns fit one
@@ -188,7 +192,7 @@ struct ResPartition {
     double cost = -1.0;  // < 0: no partition
 };
 
-inline ResPartition res_partition(int nx, int pt, int nz, int cpml, int n, int img_bytes, size_t smem_limit)
+inline ResPartition res_partition(int nx, int pt, int nz, int cpml, int n, int min_rows, int img_bytes, size_t smem_limit)
 {
     const int nzi = nz - 8, cap_u = res_row_cap(nx, pt, cpml, false, false, img_bytes, smem_limit),
               cap_1 = res_row_cap(nx, pt, cpml, false, true, img_bytes, smem_limit),
@@ -199,12 +203,12 @@ inline ResPartition res_partition(int nx, int pt, int nz, int cpml, int n, int i
     auto turns = [&](int rows) { return std::ceil(rows / lanes); };
     ResPartition best;
     for (int extra = 0; extra <= (zone ? std::min(nzi - zone, 12) : 0); extra++)
-        for (int lower = zone ? 1 : 0; lower <= (zone ? std::min(n, (zone + extra) / kResMinRows) : 0); lower++) {
+        for (int lower = zone ? 1 : 0; lower <= (zone ? std::min(n, (zone + extra) / min_rows) : 0); lower++) {
             const int upper = n - lower, rest = nzi - zone - extra;
             if ((rest == 0) != (upper == 0)) continue;
             const int umax = upper ? (rest + upper - 1) / upper : 0, lmax = lower ? (zone + extra + lower - 1) / lower : 0;
-            if (upper && (rest / upper < kResMinRows || umax > cap_u)) continue;
-            if (lower && ((zone + extra) / lower < kResMinRows || lmax > (lower == 1 ? cap_1 : cap_l))) continue;
+            if (upper && (rest / upper < min_rows || umax > cap_u)) continue;
+            if (lower && ((zone + extra) / lower < min_rows || lmax > (lower == 1 ? cap_1 : cap_l))) continue;
             const double cu = turns(umax), cl = lower ? turns(lmax) * 1.5 + turns(lower == 1 ? lmax : lmax + 8) * 0.7 + 1.5 : 0.0;
             const double c = std::max(cu, cl) + 1e-2 * (cu + cl) + 1e-3 * (umax + lmax);
             if (best.cost < 0 || c < best.cost - 1e-9) {
@@ -238,7 +242,7 @@ inline bool resident_plan(const std::vector<int> &nx, int nz, int cpml, size_t s
     int wmax = 0;
     for (int w : nx) wmax = std::max(wmax, w);
     const int pt = res_pitch(wmax, img_bytes == 0);
-    const int nb = (int)nx.size(), nzi = nz - 8, sms = std::min(n_sm, kResMaxCtas), most = std::min(sms, nzi / kResMinRows);
+    const int nb = (int)nx.size(), nzi = nz - 8, sms = std::min(n_sm, kResMaxCtas), min_rows = res_min_rows(nb), most = std::min(sms, nzi / min_rows);
     struct Width {
         int nx, least;
         std::vector<ResPartition> part;  // by CTA count
@@ -249,7 +253,7 @@ inline bool resident_plan(const std::vector<int> &nx, int nz, int cpml, size_t s
             if (x.nx == w) return x;
         Width x{w, 0, std::vector<ResPartition>(std::max(1, most + 1))};
         for (int n = 1; n <= most; n++) {
-            x.part[n] = res_partition(w, pt, nz, cpml, n, img_bytes, smem_limit);
+            x.part[n] = res_partition(w, pt, nz, cpml, n, min_rows, img_bytes, smem_limit);
             if (x.part[n].cost >= 0 && !x.least) x.least = n;
             // never a costlier split than with fewer CTAs
             if (n > 1 && x.part[n - 1].cost >= 0 && (x.part[n].cost < 0 || x.part[n].cost > x.part[n - 1].cost))

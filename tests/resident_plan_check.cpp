@@ -114,7 +114,7 @@ static bool check(const std::vector<int> &w, int nz, int cpml, int adjoint, size
             const int s = g.shot[c];
             CHECK(s < (int)w.size() && g.xs[c] < set.nshots);
             CHECK(c >= g.first[c] && c < g.first[c] + g.count[c] && g.first[c] + g.count[c] <= g.n);
-            CHECK(g.shot[g.first[c]] == s && g.nrow[c] >= (g.count[c] > 1 ? kResMinRows : 1));
+            CHECK(g.shot[g.first[c]] == s && g.nrow[c] >= (g.count[c] > 1 ? res_min_rows((int)w.size()) : 1));
             CHECK(g.row0[c] == rows[s]);
             rows[s] += g.nrow[c];
             if (c == g.first[c]) seen[s]++;
