@@ -30,7 +30,7 @@
 // residual, next u and Z, edge rows out, imaging.  A block barrier ends each part.  Arithmetic on
 // pairs of columns (FADD2, FFMA2) halves the instructions of the stencils.
 //
-// What bounds it: latency.  A C1 step (209 x 209, 100 bands of 2 rows; 2.8 us forward, 3.3 us adjoint) is 1.8 us (2.2 us
+// What bounds it: latency.  A C1 step (209 x 209; 2.75 us forward, 3.2 us adjoint) is about 1.8 us (2.2 us
 // of adjoint) of arithmetic between block barriers, about 4.5 cycles an instruction of the longest
 // thread, and 1.0 us for the exchange (a bare exchange of one row measures 0.9 - 1.1 us a step, of
 // 4 rows of 100 pairs 1.3 us, whatever the number of CTAs; flags with fences 1.7 - 2.0 us).  So: the
@@ -38,7 +38,7 @@
 // them, registers over shared memory up to the point where they spill (spills miss the small L1
 // that this much shared memory leaves), 2 columns a thread (4: C1 3.75 us an adjoint step against
 // 3.3, fewer threads a band).  A 2000-step C1 gradient with FP32 images took 16.8 ms on one 16-CTA
-// cluster, takes 12.3; 8 shots with FP16 images 36.2 -> 18.6 (two waves of clusters before); the
+// cluster, takes 11.9; 8 shots with FP16 images 36.2 -> 18.5 (two waves of clusters before); the
 // adjoint of one 609 x 309 shot 34 -> 20 ms for 3000 steps.
 #pragma once
 

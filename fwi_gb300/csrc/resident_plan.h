@@ -9,7 +9,6 @@
 
 #include <algorithm>
 #include <climits>
-#include <cmath>
 #include <cstddef>
 #include <cstdint>
 #include <vector>
@@ -192,23 +191,31 @@ struct ResPartition {
     double cost = -1.0;  // < 0: no partition
 };
 
-inline ResPartition res_partition(int nx, int pt, int nz, int cpml, int n, int min_rows, int img_bytes, size_t smem_limit)
+// What a window's CTAs can take: row segments, and rows of an upper band, of the only bottom band, of
+// one of several.
+struct ResCaps {
+    int lanes, upper, only, lower;
+};
+inline ResCaps res_caps(int nx, int pt, int cpml, int img_bytes, size_t smem_limit)
 {
-    const int nzi = nz - 8, cap_u = res_row_cap(nx, pt, cpml, false, false, img_bytes, smem_limit),
-              cap_1 = res_row_cap(nx, pt, cpml, false, true, img_bytes, smem_limit),
-              cap_l = res_row_cap(nx, pt, cpml, true, true, img_bytes, smem_limit);
-    const int zone = cpml > 4 ? std::min(nzi, cpml) : 0;
-    const double lanes = std::max(1, res_lanes(nx, pt, cpml));
+    return {std::max(1, res_lanes(nx, pt, cpml)), res_row_cap(nx, pt, cpml, false, false, img_bytes, smem_limit),
+            res_row_cap(nx, pt, cpml, false, true, img_bytes, smem_limit),
+            res_row_cap(nx, pt, cpml, true, true, img_bytes, smem_limit)};
+}
+
+inline ResPartition res_partition(const ResCaps &cap, int nz, int cpml, int n, int min_rows)
+{
+    const int nzi = nz - 8, zone = cpml > 4 ? std::min(nzi, cpml) : 0;
     // rows a thread takes in turn
-    auto turns = [&](int rows) { return std::ceil(rows / lanes); };
+    auto turns = [&](int rows) { return (double)((rows + cap.lanes - 1) / cap.lanes); };
     ResPartition best;
     for (int extra = 0; extra <= (zone ? std::min(nzi - zone, 12) : 0); extra++)
         for (int lower = zone ? 1 : 0; lower <= (zone ? std::min(n, (zone + extra) / min_rows) : 0); lower++) {
             const int upper = n - lower, rest = nzi - zone - extra;
             if ((rest == 0) != (upper == 0)) continue;
             const int umax = upper ? (rest + upper - 1) / upper : 0, lmax = lower ? (zone + extra + lower - 1) / lower : 0;
-            if (upper && (rest / upper < min_rows || umax > cap_u)) continue;
-            if (lower && ((zone + extra) / lower < min_rows || lmax > (lower == 1 ? cap_1 : cap_l))) continue;
+            if (upper && (rest / upper < min_rows || umax > cap.upper)) continue;
+            if (lower && ((zone + extra) / lower < min_rows || lmax > (lower == 1 ? cap.only : cap.lower))) continue;
             const double cu = turns(umax), cl = lower ? turns(lmax) * 1.5 + turns(lower == 1 ? lmax : lmax + 8) * 0.7 + 1.5 : 0.0;
             const double c = std::max(cu, cl) + 1e-2 * (cu + cl) + 1e-3 * (umax + lmax);
             if (best.cost < 0 || c < best.cost - 1e-9) {
@@ -252,8 +259,10 @@ inline bool resident_plan(const std::vector<int> &nx, int nz, int cpml, size_t s
         for (Width &x : widths)
             if (x.nx == w) return x;
         Width x{w, 0, std::vector<ResPartition>(std::max(1, most + 1))};
-        for (int n = 1; n <= most; n++) {
-            x.part[n] = res_partition(w, pt, nz, cpml, n, min_rows, img_bytes, smem_limit);
+        const ResCaps cap = res_caps(w, pt, cpml, img_bytes, smem_limit);
+        // a shot alone takes all it can use: only the largest counts are looked at (its plan: 0.7 -> 0.3 ms)
+        for (int n = nb == 1 ? std::max(1, most - 48) : 1; n <= most; n++) {
+            x.part[n] = res_partition(cap, nz, cpml, n, min_rows);
             if (x.part[n].cost >= 0 && !x.least) x.least = n;
             // never a costlier split than with fewer CTAs
             if (n > 1 && x.part[n - 1].cost >= 0 && (x.part[n].cost < 0 || x.part[n].cost > x.part[n - 1].cost))
