@@ -1343,8 +1343,10 @@ template <typename T> struct Ctx : CtxBase {
     {
         run = ResidentRun();
         if (sizeof(T) != 4 || !use_tma) return false;
-        if (const char *e = getenv("FWI_CLUSTER"))
-            if (atoi(e) == 0) return false;
+        // FWI_CLUSTER=0: the per-step passes; FWI_RESIDENT=0: the cluster path where it fits (tests)
+        for (const char *name : {"FWI_CLUSTER", "FWI_RESIDENT"})
+            if (const char *e = getenv(name))
+                if (atoi(e) == 0) return false;
         const bool ckpt = want_grad && cfg.store == FWI_STORE_CHECKPOINT;
         const bool full = want_grad && cfg.store == FWI_STORE_FULL;
         if (want_grad && !full && !ckpt) return false;
@@ -1419,7 +1421,7 @@ template <typename T> struct Ctx : CtxBase {
                 a.period = period;
                 a.load_ck = load_ck;
                 a.save_ck = save_ck;
-                a.tile_order = !cluster_path(nxm);
+                a.order = cluster_path(nxm) ? fwi::kResAsCluster : b.inline_strip ? fwi::kResAsInline : fwi::kResAsStrip;
                 a.plain_images = cfg.mode != FWI_MODE_EXACT;
                 a.ck = ck;
                 a.ck_stride = (long)B * slot;

@@ -103,6 +103,10 @@ __device__ __forceinline__ float2 add(const float2 &x, const float2 &y) { return
 __device__ __forceinline__ float2 mul(const float2 &x, const float2 &y) { return __fmul2_rn(x, y); }
 __device__ __forceinline__ float2 fma(const float2 &x, const float2 &y, const float2 &z) { return __ffma2_rn(x, y, z); }
 __device__ __forceinline__ float2 scaled(const float2 &x, float v) { return __fmul2_rn(x, both(v)); }
+// A product that goes into a sum rounded, as the sum is.  A packed product with one use is merged into the
+// packed sum that takes it (one rounding, whatever the intrinsics' names say: measured on every such
+// form); of scalars it is not.
+__device__ __forceinline__ float2 rounded(const float2 &x, float v) { return make_float2(__fmul_rn(x.x, v), __fmul_rn(x.y, v)); }
 // the columns below nval, zero from there on (nval >= 1)
 __device__ __forceinline__ float2 keep(const float2 &v, int nval) { return make_float2(v.x, nval > 1 ? v.y : 0.f); }
 
@@ -131,21 +135,22 @@ __device__ __forceinline__ float2 res_diff(const float2 &p, const float2 &m)
 }
 
 // The memory variables' updates, psi' = b psi + a D and zeta' = b zeta + a (d2 + D), D = d1 inv_dh,
-// and the layer's term D + zeta'.  The compiler contracts the cluster path's expressions and the
-// tile passes' differently; a batch rounds as the path that would otherwise take it (`tile`: as the
-// tile passes), so that its forward is that path's bit for bit.
-__device__ __forceinline__ float2 res_psi(bool tile, const float2 &b, const float2 &psi, const float2 &a, const float2 &D)
+// and the layer's term D + zeta'.  nvcc contracts these sums in one way in the cluster kernels, in another
+// in the layer tiles, and psi_x in a third in the strip pass; a batch rounds as the path that would
+// otherwise take it (ResOrder), so that its traces and images are that path's bit for bit: a last-bit
+// difference turns into one of 2^-8 where a BF16 image falls on the other side of a rounding boundary.
+__device__ __forceinline__ float2 res_psi(bool strip, const float2 &b, const float2 &psi, const float2 &a, const float2 &D)
 {
-    return tile ? fma(a, D, mul(b, psi)) : fma(b, psi, mul(a, D));
+    return strip ? fma(a, D, mul(b, psi)) : fma(b, psi, mul(a, D));
 }
 __device__ __forceinline__ float2 res_zeta(bool tile, const float2 &b, const float2 &zeta, const float2 &a,
                                            const float2 &d2, const float2 &d1, float inv_dh)
 {
-    return fma(b, zeta, mul(a, tile ? fma(d1, both(inv_dh), d2) : add(d2, scaled(d1, inv_dh))));
+    return fma(b, zeta, mul(a, tile ? fma(d1, both(inv_dh), d2) : add(d2, rounded(d1, inv_dh))));
 }
 __device__ __forceinline__ float2 res_term(bool tile, const float2 &d1, float inv_dh, const float2 &zeta)
 {
-    return tile ? fma(d1, both(inv_dh), zeta) : add(scaled(d1, inv_dh), zeta);
+    return tile ? fma(d1, both(inv_dh), zeta) : add(rounded(d1, inv_dh), zeta);
 }
 
 // Derivatives of 2 columns, along z from 9 rows, along x from the 10 values at p - 4 .. p + 5.
@@ -433,7 +438,7 @@ k_resident_fwd(const __grid_constant__ Batch<float> b, const __grid_constant__ R
     __syncthreads();
     res_tables(b, B, S.ax, S.bx, S.az - kRad, S.bz - kRad);
     const float inv_dh = b.inv_dh, inv_dh2 = b.inv_dh2;
-    const bool tile = a.tile_order, plain = a.plain_images;
+    const bool tile = a.order != kResAsCluster, strip = a.order == kResAsStrip, plain = a.plain_images;
     const long so = (long)B.s * b.slot;
     const int r0 = B.seg * B.rows, nr = B.use ? min(B.rows, nrow - r0) : 0;  // the thread's rows [r0, r0 + nr)
     const int nval = min(2, B.nx - 4 - ix);                                   // its interior columns
@@ -515,13 +520,13 @@ k_resident_fwd(const __grid_constant__ Batch<float> b, const __grid_constant__ R
             const float2 ax = ld2(S.ax + cx), bx = ld2(S.bx + cx);
             for (int rr = 0; rr < nr; rr++) {
                 float *const ps = pS + rr * SD * WB;
-                put2(ps, keep(res_psi(tile, bx, ld2(ps), ax, scaled(ResWindow(pc + rr * OWN * PT).d1(), inv_dh)), nval));
+                put2(ps, keep(res_psi(strip, bx, ld2(ps), ax, scaled(ResWindow(pc + rr * OWN * PT).d1(), inv_dh)), nval));
             }
             res_side_sync(B);
             // what they add to Dxx P: zeta_x and Dx psi_x (in the bottom layer also where only psi_x reaches)
             for (int rr = 0; rr < nr; rr++) {
                 float *const ps = pS + rr * SD * WB;
-                const float2 gp = scaled(ResWindow(pc + rr * OWN * PT).d2(), inv_dh2);
+                const float2 gp = rounded(ResWindow(pc + rr * OWN * PT).d2(), inv_dh2);
                 const float2 dx = ResWindow(ps).d1();
                 const float2 z = keep(res_zeta(tile, bx, ld2(ps + WB), ax, gp, dx, inv_dh), nval);
                 const float2 d = res_term(tile, dx, inv_dh, z);
@@ -598,7 +603,7 @@ k_resident_fwd(const __grid_constant__ Batch<float> b, const __grid_constant__ R
                 win[rr + 8] = ld2(fc + (rr + 4) * PT);
                 const float *const o = pO + rr * OWN * PT;
                 const ResWindow w(pc + rr * OWN * PT);
-                const float2 G0 = scaled(w.d2(), inv_dh2), H0 = scaled(res_d2z(win + rr), inv_dh2);
+                const float2 G0 = rounded(w.d2(), inv_dh2), H0 = rounded(res_d2z(win + rr), inv_dh2);
                 float2 G = G0, H = H0;
                 if (B.side) G = add(G, ld2(pS + (rr * SD + 2) * WB));
                 if (B.bottom) H = add(H, ld2(S.zo + ((r0 + rr) * 2 + 1) * PT + ix));

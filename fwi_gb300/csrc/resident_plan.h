@@ -70,6 +70,10 @@ struct ResidentSet {
     size_t smem;
 };
 
+// Whose roundings of the CPML terms a forward launch follows: the cluster path's, those of the layer tiles
+// that advance psi themselves, those of the layer tiles after the strip pass.
+enum ResOrder { kResAsCluster, kResAsInline, kResAsStrip };
+
 // Arguments of one forward launch: global steps [g0, g1) of a batch whose clock runs to ntb.
 struct ResFwdArgs {
     int ntb, g0, g1;
@@ -77,7 +81,7 @@ struct ResFwdArgs {
     int period;      // g - seg period + (seg & 1) period of step g, seg = g / period (nt_max: slot g)
     int load_ck;     // checkpoint to start from, or -1: zero state
     int save_ck;     // checkpoints 0 .. save_ck - 1 are written (step k period)
-    int tile_order;  // CPML terms rounded as the tile passes', else as the cluster path's
+    int order;       // ResOrder: the path this batch would otherwise take
     int plain_images;  // images of the plain stencils (reference mode)
     float *ck;       // [checkpoint][8][ck_stride]
     long ck_stride;
