@@ -318,48 +318,11 @@ template <typename T> struct alignas(16) Pack {
 
 // The passes of the L-BFGS recursion below: sums and coefficients are FP64, whose pipe takes 64 cycles
 // a warp instruction on an SM quarter, conversions from and to FP32 included (an axpy with a dot, 7 such
-// operations a value, was bound by them: 75 us for 3 x 1.6 M values).  So: FP32 widens by integer
-// operations, x + k u is rounded from error-free FP32 parts, no FP64 operation by 1 or 0; copies made by
+// operations a value, was bound by them: 75 us for 3 x 1.6 M values).  So: values widen and narrow by
+// integer operations, no FP64 operation by 1 or 0, which leaves two multiply-adds a value; copies made by
 // the pass that has the values, scalar steps by the last block of the reduction that feeds them.
 // First step and 5 directions and updates on 2009 x 809: 4.90 ms before, 3.37 with FP64
-// conversions in 2 blocks an SM, 1.8 now.
-
-// The rare case, out of line: as a branch the compiler would run its FP64 operations for every value.
-__device__ __noinline__ float axpy_any(float x, float u, double k) { return (float)((double)x + k * (double)u); }
-
-// An FP64 coefficient, for FP32 operands in two parts (48 bits) when it lies well inside FP32's range.
-template <typename T> struct LbCoef {
-    double k;
-    __device__ __forceinline__ explicit LbCoef(double k_) : k(k_) {}
-    __device__ __forceinline__ T axpy(T x, T u) const { return x + k * u; }
-    __device__ __forceinline__ T scale(T x) const { return k * x; }
-};
-template <> struct LbCoef<float> {
-    double k;
-    float h, l;
-    bool parts;
-    __device__ __forceinline__ explicit LbCoef(double k_) : k(k_), h((float)k_)
-    {
-        l = (float)(k - (double)h);
-        parts = fabs(k) < 1e30 && (fabs(k) > 1e-20 || k == 0.0);
-    }
-    // x + k u rounded once, to within 2^-20 of a last place of FP64's value: the product and the sum
-    // with their exact errors (fused multiply-add; Knuth's two-sum), then one rounding.  Where a part
-    // could underflow or overflow, in FP64.
-    __device__ __forceinline__ float axpy(float x, float u) const
-    {
-        const float p = h * u, e = __fmaf_rn(h, u, -p), s = x + p, t = s - x;
-        const float r = s + (((x - (s - t)) + (p - t)) + __fmaf_rn(l, u, e));
-        if (parts && fabsf(r) <= 3e38f && (fmaxf(fabsf(p), fabsf(x)) > 0x1p-70f || u == 0.f)) return r;
-        return axpy_any(x, u, k);
-    }
-    __device__ __forceinline__ float scale(float x) const
-    {
-        const float p = h * x, r = p + __fmaf_rn(l, x, __fmaf_rn(h, x, -p));
-        if (parts && fabsf(r) <= 3e38f && (fabsf(p) > 0x1p-70f || x == 0.f)) return r;
-        return axpy_any(0.f, x, k);
-    }
-};
+// conversions in 2 blocks an SM, 1.89 now.
 
 // Scalars of the two-loop recursion.
 struct LbScalars {
@@ -473,8 +436,7 @@ __global__ void __launch_bounds__(kRedThreads) k_lb_axpy_dot(Tri<T> x, CTri<T> s
 {
     using P = Pack<T>;
     double v[1][3] = {};
-    const LbCoef<T> k1[3] = {LbCoef<T>(S->coefB[0]), LbCoef<T>(S->coefB[1]), LbCoef<T>(S->coefB[2])};
-    const LbCoef<T> gam[3] = {LbCoef<T>(S->coefA[0]), LbCoef<T>(S->coefA[1]), LbCoef<T>(S->coefA[2])};
+    const double k1[3] = {S->coefB[0], S->coefB[1], S->coefB[2]}, gam[3] = {S->coefA[0], S->coefA[1], S->coefA[2]};
     for (long i = P::N * (blockIdx.x * (long)blockDim.x + threadIdx.x); i < n; i += P::N * (long)gridDim.x * blockDim.x)
 #pragma unroll
         for (int p = 0; p < 3; p++) {
@@ -484,8 +446,8 @@ __global__ void __launch_bounds__(kRedThreads) k_lb_axpy_dot(Tri<T> x, CTri<T> s
             if (AFTER != LB_LAST) nv = P::get(next.p[p] + i);
 #pragma unroll
             for (int q = 0; q < P::N; q++) {
-                xv.v[q] = k1[p].axpy(xv.v[q], uv.v[q]);
-                if (GAMMA) xv.v[q] = gam[p].scale(xv.v[q]);
+                xv.v[q] = fwi::narrow<T>(__fma_rn(k1[p], fwi::widen(uv.v[q]), fwi::widen(xv.v[q])));
+                if (GAMMA) xv.v[q] = fwi::narrow<T>(gam[p] * fwi::widen(xv.v[q]));
                 if (AFTER != LB_LAST) v[0][p] += fwi::widen(nv.v[q]) * fwi::widen(xv.v[q]);
             }
             xv.put(x.p[p] + i);
