@@ -1266,6 +1266,7 @@ template <typename T> struct Ctx : CtxBase {
     };
     static constexpr size_t kResidentPlans = 8;
     std::vector<std::unique_ptr<ResidentPlan>> resident_plans;  // least recently used first
+    fwi::ResWidths resident_widths;
     uint64_t *res_x = nullptr, *res_w = nullptr;  // exchanged rows and maxima (zeroed when made)
     size_t res_words = 0;                         // words of the exchanged rows
     unsigned res_tag = 1;                         // the next unused step tag
@@ -1282,7 +1283,7 @@ template <typename T> struct Ctx : CtxBase {
         std::unique_ptr<ResidentPlan> p(new ResidentPlan);
         p->windows = windows;
         p->img_bytes = img_bytes;
-        if (!fwi::resident_plan(windows, nz, cfg.cpml, smem, n_sm, img_bytes, p->sets)) p->sets.clear();
+        if (!fwi::resident_plan(windows, nz, cfg.cpml, smem, n_sm, img_bytes, p->sets, &resident_widths)) p->sets.clear();
         resident_plans.push_back(std::move(p));
         const std::vector<fwi::ResidentSet> &sets = resident_plans.back()->sets;
         return sets.empty() ? nullptr : &sets;

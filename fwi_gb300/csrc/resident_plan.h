@@ -11,6 +11,7 @@
 #include <climits>
 #include <cstddef>
 #include <cstdint>
+#include <map>
 #include <vector>
 
 #include "common.cuh"
@@ -207,28 +208,48 @@ inline ResCaps res_caps(int nx, int pt, int cpml, int img_bytes, size_t smem_lim
             res_row_cap(nx, pt, cpml, true, true, img_bytes, smem_limit)};
 }
 
-inline ResPartition res_partition(const ResCaps &cap, int nz, int cpml, int n, int min_rows)
+// The cheapest partition into at most n CTAs, for every n to `most`.  A cost depends on the tallest upper
+// and the tallest lower band only, so that for each of these heights the fewest CTAs are tried (a few
+// hundred partitions; all counts and splits, a thousand times as many, took 0.3 ms a width).
+inline std::vector<ResPartition> res_partitions(const ResCaps &cap, int nz, int cpml, int most, int min_rows)
 {
     const int nzi = nz - 8, zone = cpml > 4 ? std::min(nzi, cpml) : 0;
+    std::vector<ResPartition> best(std::max(1, most + 1));
     // rows a thread takes in turn
     auto turns = [&](int rows) { return (double)((rows + cap.lanes - 1) / cap.lanes); };
-    ResPartition best;
-    for (int extra = 0; extra <= (zone ? std::min(nzi - zone, 12) : 0); extra++)
-        for (int lower = zone ? 1 : 0; lower <= (zone ? std::min(n, (zone + extra) / min_rows) : 0); lower++) {
-            const int upper = n - lower, rest = nzi - zone - extra;
-            if ((rest == 0) != (upper == 0)) continue;
-            const int umax = upper ? (rest + upper - 1) / upper : 0, lmax = lower ? (zone + extra + lower - 1) / lower : 0;
-            if (upper && (rest / upper < min_rows || umax > cap.upper)) continue;
-            if (lower && ((zone + extra) / lower < min_rows || lmax > (lower == 1 ? cap.only : cap.lower))) continue;
-            const double cu = turns(umax), cl = lower ? turns(lmax) * 1.5 + turns(lower == 1 ? lmax : lmax + 8) * 0.7 + 1.5 : 0.0;
-            const double c = std::max(cu, cl) + 1e-2 * (cu + cl) + 1e-3 * (umax + lmax);
-            if (best.cost < 0 || c < best.cost - 1e-9) {
-                best.upper = upper;
-                best.lower = lower;
-                best.extra = extra;
-                best.cost = c;
+    auto tallest = [](int rows, int n) { return (rows + n - 1) / n; };
+    for (int extra = 0; extra <= (zone ? std::min(nzi - zone, 12) : 0); extra++) {
+        const int low = zone + (zone ? extra : 0), rest = nzi - low;
+        for (int lower = zone ? 1 : 0, next; lower <= (zone ? std::min(most, low / min_rows) : 0); lower = next) {
+            const int lmax = lower ? tallest(low, lower) : 0;
+            // the next count with a lower tallest band (one bottom band costs otherwise than several)
+            next = lower <= 1 ? lower + 1 : lmax > 1 ? tallest(low, lmax - 1) : most + 1;
+            if (lmax > (lower == 1 ? cap.only : cap.lower)) continue;
+            const double cl = lower ? turns(lmax) * 1.5 + turns(lower == 1 ? lmax : lmax + 8) * 0.7 + 1.5 : 0.0;
+            auto offer = [&](int upper, int umax) {
+                if (upper + lower < 1 || upper + lower > most) return;
+                const double cu = turns(umax), c = std::max(cu, cl) + 1e-2 * (cu + cl) + 1e-3 * (umax + lmax);
+                ResPartition &p = best[upper + lower];
+                if (p.cost >= 0 && c >= p.cost - 1e-9) return;
+                p.upper = upper;
+                p.lower = lower;
+                p.extra = extra;
+                p.cost = c;
+            };
+            if (rest == 0) {
+                offer(0, 0);
+                continue;
+            }
+            for (int umax = std::min(cap.upper, rest); umax >= 1;) {
+                const int upper = tallest(rest, umax);
+                if (rest / upper < min_rows || upper + lower > most) break;
+                offer(upper, tallest(rest, upper));
+                umax = tallest(rest, upper) - 1;
             }
         }
+    }
+    for (int n = 1; n <= most; n++)
+        if (best[n - 1].cost >= 0 && (best[n].cost < 0 || best[n].cost > best[n - 1].cost)) best[n] = best[n - 1];
     return best;
 }
 
@@ -242,74 +263,73 @@ inline std::vector<int> res_bands(const ResPartition &p, int nz, int cpml)
     return r;
 }
 
+// The partitions of a window's width, and those of the widths seen so far, which a context keeps for its
+// grid (about kResWidths at most; 10 to 25 microseconds a width to make).
+struct ResWidth {
+    int least = 0;                   // the fewest CTAs that hold the window (0: none do)
+    std::vector<ResPartition> part;  // by CTA count
+    std::vector<int> more;           // the next count that lowers the cost (past the last: none)
+};
+using ResWidths = std::map<long, ResWidth>;
+constexpr size_t kResWidths = 512;
+
 // The launches of a batch whose shots have windows nx[0], nx[1], ...: consecutive shots share a
 // launch while their fewest CTAs fit on n_sm SMs (windows of one width: the same number in each),
 // then the SMs left go one by one to the shot with the costliest band.  False if some window does
-// not fit at all.
+// not fit at all.  `kept`: the widths of earlier plans for the same grid, layer, limit and SMs.
 inline bool resident_plan(const std::vector<int> &nx, int nz, int cpml, size_t smem_limit, int n_sm, int img_bytes,
-                          std::vector<ResidentSet> &out)
+                          std::vector<ResidentSet> &out, ResWidths *kept = nullptr)
 {
     out.clear();
     int wmax = 0;
     for (int w : nx) wmax = std::max(wmax, w);
     const int pt = res_pitch(wmax, img_bytes == 0);
     const int nb = (int)nx.size(), nzi = nz - 8, sms = std::min(n_sm, kResMaxCtas), min_rows = res_min_rows(nb), most = std::min(sms, nzi / min_rows);
-    struct Width {
-        int nx, least;
-        std::vector<ResPartition> part;  // by CTA count
-    };
-    std::vector<Width> widths;
-    auto width = [&](int w) -> Width & {
-        for (Width &x : widths)
-            if (x.nx == w) return x;
-        Width x{w, 0, std::vector<ResPartition>(std::max(1, most + 1))};
-        const ResCaps cap = res_caps(w, pt, cpml, img_bytes, smem_limit);
-        // a shot alone takes all it can use: only the largest counts are looked at (its plan: 0.7 -> 0.3 ms)
-        for (int n = nb == 1 ? std::max(1, most - 48) : 1; n <= most; n++) {
-            x.part[n] = res_partition(cap, nz, cpml, n, min_rows);
-            if (x.part[n].cost >= 0 && !x.least) x.least = n;
-            // never a costlier split than with fewer CTAs
-            if (n > 1 && x.part[n - 1].cost >= 0 && (x.part[n].cost < 0 || x.part[n].cost > x.part[n - 1].cost))
-                x.part[n] = x.part[n - 1];
-        }
-        widths.push_back(x);
-        return widths.back();
-    };
+    if (nzi < 1) return false;
+    ResWidths own, &widths = kept ? *kept : own;
+    if (widths.size() > kResWidths) widths.clear();
+    std::vector<const ResWidth *> of(nb);  // each shot's
     bool uniform = true;
-    for (int w : nx) {
-        if (width(w).least == 0) return false;
-        uniform = uniform && w == nx[0];
+    for (int k = 0; k < nb; k++) {
+        ResWidth &x = widths[(long)nx[k] << 32 | pt << 8 | img_bytes << 4 | min_rows];
+        if (x.part.empty()) {
+            x.part = res_partitions(res_caps(nx[k], pt, cpml, img_bytes, smem_limit), nz, cpml, most, min_rows);
+            for (int n = 1; n <= most && !x.least; n++)
+                if (x.part[n].cost >= 0) x.least = n;
+            x.more.assign(most + 2, most + 1);
+            for (int n = most - 1; n >= 1; n--) x.more[n] = x.part[n + 1].cost < x.part[n].cost ? n + 1 : x.more[n + 1];
+        }
+        if (!x.least) return false;
+        of[k] = &x;
+        uniform = uniform && nx[k] == nx[0];
     }
     int per = nb;
     if (uniform) {
-        const int fit = sms / width(nx[0]).least, sets = (nb + fit - 1) / fit;
+        const int fit = sms / of[0]->least, sets = (nb + fit - 1) / fit;
         per = (nb + sets - 1) / sets;
     }
     for (int s0 = 0; s0 < nb;) {
         int s1 = s0, used = 0;
         std::vector<int> n;
-        while (s1 < nb && s1 - s0 < per && used + width(nx[s1]).least <= sms) {
-            n.push_back(width(nx[s1]).least);
+        while (s1 < nb && s1 - s0 < per && used + of[s1]->least <= sms) {
+            n.push_back(of[s1]->least);
             used += n.back();
             s1++;
         }
         for (;;) {  // the SMs left
-            int pick = -1, to = 0;
+            int pick = -1;
             double worst = 0.0;
             for (int k = 0; k < (int)n.size(); k++) {
-                const Width &w = width(nx[s0 + k]);
-                int m = n[k] + 1;  // the next count that lowers this shot's cost
-                while (m <= most && w.part[m].cost >= w.part[n[k]].cost) m++;
-                if (m > most || used + m - n[k] > sms) continue;
-                if (pick < 0 || w.part[n[k]].cost > worst) {
-                    pick = k;
-                    to = m;
-                    worst = w.part[n[k]].cost;
-                }
+                const ResWidth &w = *of[s0 + k];
+                const int m = w.more[n[k]];
+                if (m > most || used + m - n[k] > sms || (pick >= 0 && w.part[n[k]].cost <= worst)) continue;
+                pick = k;
+                worst = w.part[n[k]].cost;
             }
             if (pick < 0) break;
-            used += to - n[pick];
-            n[pick] = to;
+            const int m = of[s0 + pick]->more[n[pick]];
+            used += m - n[pick];
+            n[pick] = m;
         }
         ResidentSet set{};
         set.nshots = s1 - s0;
@@ -318,7 +338,7 @@ inline bool resident_plan(const std::vector<int> &nx, int nz, int cpml, size_t s
         int c = 0;
         for (int k = 0; k < set.nshots; k++) {
             const int w = nx[s0 + k], first = c;
-            const std::vector<int> bands = res_bands(width(w).part[n[k]], nz, cpml);
+            const std::vector<int> bands = res_bands(of[s0 + k]->part[n[k]], nz, cpml);
             int row = 0;
             for (int r : bands) {
                 g.shot[c] = (unsigned short)(s0 + k);
