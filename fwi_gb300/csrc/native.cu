@@ -666,26 +666,99 @@ struct CtxBase {
     }
 };
 
-// One batch at a time on the resident path of a device, over every context of the process: the
-// CTAs of such a launch wait on one another, so no two launches may hold part of the SMs each.
-// Given back when the stream's work is done.
-std::mutex &resident_mutex(int device)
-{
-    static std::mutex mu[64];
-    return mu[device & 63];
-}
-struct ResidentTurn {
-    std::mutex *mu;
-    cudaStream_t st;
-    ResidentTurn(std::mutex *m, cudaStream_t s) : mu(m), st(s)
+// The resident path of a device, over every context of the process.  The CTAs of a resident launch wait on
+// one another, one to an SM, so that the launches in flight never want more SMs than there are.  Batches
+// in flight at the same time plan for equal shares of the SMs (a plan's CTAs do not change its results)
+// and run side by side: 4 contexts in 4 threads, one C1 shot each, take 13.0 ms a call of each, 47 where
+// every batch had the whole device in turn, 16.9 on the cluster path.
+struct ResidentQueue {
+    struct Phase {  // the launches of a batch's forward or adjoint, one after another
+        cudaEvent_t done;
+        cudaStream_t st;
+        int ctas;  // of the largest
+    };
+    std::mutex mu;
+    std::vector<struct ResidentBatch *> batches;  // in flight
+    std::vector<Phase> phases;                    // issued and perhaps not done, oldest first
+
+    // A phase about to be issued: it runs beside the newest phases that leave it its SMs, one of a stream
+    // at a time, and waits for the older ones.  So whatever runs together had room, counted by the newest.
+    cudaError_t enter(const Phase &p, int n_sm)
     {
-        if (mu) mu->lock();
+        leave(p.done);
+        phases.erase(std::remove_if(phases.begin(), phases.end(),
+                                    [](const Phase &o) {
+                                        const bool done = cudaEventQuery(o.done) == cudaSuccess;
+                                        if (!done) cudaGetLastError();  // (not ready)
+                                        return done;
+                                    }),
+                     phases.end());
+        size_t k = phases.size();
+        for (int used = p.ctas; k > 0; k--) {
+            const Phase &o = phases[k - 1];
+            int counted = o.st == p.st ? o.ctas : 0;  // what its stream already counts for
+            for (size_t i = k; i < phases.size(); i++)
+                if (phases[i].st == o.st) counted = std::max(counted, phases[i].ctas);
+            used += std::max(0, o.ctas - counted);
+            if (used > n_sm) break;
+        }
+        for (size_t i = 0; i < k; i++)
+            if (const cudaError_t e = cudaStreamWaitEvent(p.st, phases[i].done, 0)) return e;
+        return cudaSuccess;
+    }
+    void leave(cudaEvent_t done)
+    {
+        phases.erase(std::remove_if(phases.begin(), phases.end(), [=](const Phase &p) { return p.done == done; }), phases.end());
+    }
+};
+ResidentQueue &resident_queue(int device)
+{
+    static ResidentQueue *const q = new ResidentQueue[64];  // (outlives every context)
+    return q[device & 63];
+}
+
+// A batch of any path, counted while it is in flight.  It shares the device with the batches in flight
+// when it begins, or with the most that its context's last batch ran beside: threads that call in turn
+// have gaps between their batches.
+struct ResidentBatch {
+    ResidentQueue &q;
+    int &last;    // of the context: the most batches in flight during its last one
+    int sharing;  // this one counted
+    int peak;
+    ResidentBatch(ResidentQueue &queue, int &last_peak) : q(queue), last(last_peak)
+    {
+        std::lock_guard<std::mutex> lock(q.mu);
+        q.batches.push_back(this);
+        peak = (int)q.batches.size();
+        for (ResidentBatch *b : q.batches) b->peak = std::max(b->peak, peak);
+        sharing = std::max(peak, last);
+    }
+    ~ResidentBatch()
+    {
+        std::lock_guard<std::mutex> lock(q.mu);
+        q.batches.erase(std::find(q.batches.begin(), q.batches.end(), this));
+        last = peak;
+    }
+    ResidentBatch(const ResidentBatch &) = delete;
+    ResidentBatch &operator=(const ResidentBatch &) = delete;
+};
+
+// Issues a phase (the device queue's lock is held meanwhile, the device not waited for).
+struct ResidentTurn {
+    ResidentQueue &q;
+    ResidentQueue::Phase phase;
+    cudaError_t err;
+    ResidentTurn(ResidentQueue &queue, cudaStream_t st, cudaEvent_t done, int ctas, int n_sm) : q(queue), phase{done, st, ctas}
+    {
+        q.mu.lock();
+        // (its last phase was a batch ago, done unless that batch ended in an error)
+        err = cudaEventSynchronize(done);
+        if (err == cudaSuccess) err = q.enter(phase, n_sm);
     }
     ~ResidentTurn()
     {
-        if (!mu) return;
-        cudaStreamSynchronize(st);
-        mu->unlock();
+        if (err == cudaSuccess && cudaEventRecord(phase.done, phase.st) == cudaSuccess) q.phases.push_back(phase);
+        q.mu.unlock();
     }
     ResidentTurn(const ResidentTurn &) = delete;
     ResidentTurn &operator=(const ResidentTurn &) = delete;
@@ -908,6 +981,13 @@ template <typename T> struct Ctx : CtxBase {
         for (void *p : allocs) cudaFree(p);
         for (const TileListEntry &e : tile_lists) cudaFree(e.dev);
         if (res_x) cudaFree(res_x);
+        for (cudaEvent_t e : ev_res)
+            if (e) {
+                ResidentQueue &rq = resident_queue(cfg.device);
+                std::lock_guard<std::mutex> lock(rq.mu);
+                rq.leave(e);
+                cudaEventDestroy(e);
+            }
         free_observed();  // (the store's scratch and the kept model are among allocs)
         if (ss.side) cudaStreamSynchronize(ss.side);
         if (rst) cudaStreamSynchronize(rst);
@@ -976,6 +1056,7 @@ template <typename T> struct Ctx : CtxBase {
             TRY(cudaStreamCreateWithPriority(&ss.side, cudaStreamNonBlocking, hi));
             TRY(cudaEventCreateWithFlags(&ss.fork, cudaEventDisableTiming));
             TRY(cudaEventCreateWithFlags(&ss.join, cudaEventDisableTiming));
+            for (cudaEvent_t &e : ev_res) TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }
         for (T **p : {&vh, &vp, &vn, &mh, &mp, &mn}) TRY(alloc(p, mslot));
         TRY(alloc(&cpa, cfg.cpml + 1));
@@ -1254,39 +1335,46 @@ template <typename T> struct Ctx : CtxBase {
 
     // The launches of a batch on the resident path (resident_plan.h): of its forward steps, of its
     // adjoint iterations; null: that phase runs otherwise.
+    using ResidentSets = std::shared_ptr<const std::vector<fwi::ResidentSet>>;
     struct ResidentRun {
-        const std::vector<fwi::ResidentSet> *fwd = nullptr, *adj = nullptr;
+        ResidentSets fwd, adj;
         bool any() const { return fwd || adj; }
+        int ctas(bool adjoint) const  // of the largest launch (an adjoint's include the recompute's)
+        {
+            int n = 0;
+            for (const auto *sets : {fwd.get(), adjoint ? adj.get() : nullptr})
+                for (size_t k = 0; sets && k < sets->size(); k++) n = std::max(n, (*sets)[k].grid.n);
+            return n;
+        }
     };
     // Plans made for the windows of recent batches (a plan is a small search on the host).
     struct ResidentPlan {
         std::vector<int> windows;
         int img_bytes = 0;  // of the images an adjoint reads; 0: forward
-        std::vector<fwi::ResidentSet> sets;
+        int sms = 0;
+        ResidentSets sets;  // null: the windows do not fit
     };
     static constexpr size_t kResidentPlans = 8;
-    std::vector<std::unique_ptr<ResidentPlan>> resident_plans;  // least recently used first
+    std::vector<ResidentPlan> resident_plans;  // least recently used first
     fwi::ResWidths resident_widths;
     uint64_t *res_x = nullptr, *res_w = nullptr;  // exchanged rows and maxima (zeroed when made)
     size_t res_words = 0;                         // words of the exchanged rows
     unsigned res_tag = 1;                         // the next unused step tag
+    int res_sharing = 1;                          // the most batches in flight during the last one (ResidentBatch)
+    cudaEvent_t ev_res[2] = {};                   // the ends of a batch's forward and adjoint phases (ResidentQueue)
 
-    const std::vector<fwi::ResidentSet> *resident_sets(const std::vector<int> &windows, int img_bytes, size_t smem)
+    ResidentSets resident_sets(const std::vector<int> &windows, int img_bytes, size_t smem, int sms)
     {
         for (size_t k = 0; k < resident_plans.size(); k++)
-            if (resident_plans[k]->img_bytes == img_bytes && resident_plans[k]->windows == windows) {
+            if (resident_plans[k].img_bytes == img_bytes && resident_plans[k].sms == sms && resident_plans[k].windows == windows) {
                 std::rotate(resident_plans.begin() + k, resident_plans.begin() + k + 1, resident_plans.end());
-                const std::vector<fwi::ResidentSet> &sets = resident_plans.back()->sets;
-                return sets.empty() ? nullptr : &sets;
+                return resident_plans.back().sets;
             }
         if (resident_plans.size() >= kResidentPlans) resident_plans.erase(resident_plans.begin());
-        std::unique_ptr<ResidentPlan> p(new ResidentPlan);
-        p->windows = windows;
-        p->img_bytes = img_bytes;
-        if (!fwi::resident_plan(windows, nz, cfg.cpml, smem, n_sm, img_bytes, p->sets, &resident_widths)) p->sets.clear();
-        resident_plans.push_back(std::move(p));
-        const std::vector<fwi::ResidentSet> &sets = resident_plans.back()->sets;
-        return sets.empty() ? nullptr : &sets;
+        auto sets = std::make_shared<std::vector<fwi::ResidentSet>>();
+        if (!fwi::resident_plan(windows, nz, cfg.cpml, smem, sms, img_bytes, *sets, &resident_widths)) sets.reset();
+        resident_plans.push_back({windows, img_bytes, sms, sets});
+        return sets;
     }
 
     // Which phases of a batch run resident on chip (prop_resident.cuh): FP32, windows that fit, and
@@ -1302,7 +1390,9 @@ template <typename T> struct Ctx : CtxBase {
     //  - Adjoint of stored images: windows to 400 wide; to 640 where all shots run at once.  Tiles ->
     //    resident: 40 of 320 x 300 11.9 -> 8.1 (200 steps), one 609 x 309 3.4 -> 2.0, three (two
     //    launches) 6.0 -> 6.4 (300 and 400 steps).
-    bool resident_path(const std::vector<DevShot> &bs, int nxm, bool want_grad, ResidentRun &run)
+    // The path does not depend on what else is in flight; with `sharing` batches in flight on the device
+    // the launches plan for that share of its SMs, or the largest of more that holds them.
+    bool resident_path(const std::vector<DevShot> &bs, int nxm, bool want_grad, int sharing, ResidentRun &run)
     {
         run = ResidentRun();
         if (sizeof(T) != 4 || !use_tma) return false;
@@ -1324,18 +1414,23 @@ template <typename T> struct Ctx : CtxBase {
         const bool fwd = nxm <= 256 || (nxm <= 400 && points <= 2000000L);
         const size_t lim = fwd || nxm <= 640 ? fwi::resident_smem_limit() : 0;
         if (!lim) return false;
-        if (fwd) run.fwd = resident_sets(w, 0, lim);
-        if (full ? nxm <= 640 : ckpt && run.fwd) run.adj = resident_sets(w, (int)store_elem(), lim);
+        if (fwd) run.fwd = resident_sets(w, 0, lim, n_sm);
+        if (full ? nxm <= 640 : ckpt && run.fwd) run.adj = resident_sets(w, (int)store_elem(), lim, n_sm);
         if (run.adj && nxm > 400 && run.adj->size() > 1) run.adj = nullptr;
         if (ckpt && !run.adj) run.fwd = nullptr;
         if (!run.any()) return false;
+        for (int share = sharing; share > 1; share--) {
+            ResidentRun part;
+            if (run.fwd) part.fwd = resident_sets(w, 0, lim, n_sm / share);
+            if (run.adj) part.adj = resident_sets(w, (int)store_elem(), lim, n_sm / share);
+            if (!part.fwd != !run.fwd || !part.adj != !run.adj) continue;
+            run = part;
+            break;
+        }
         size_t words = 0;
-        auto need = [&](const std::vector<fwi::ResidentSet> *sets) {
+        for (const auto *sets : {run.fwd.get(), run.adj.get()})
             for (size_t k = 0; sets && k < sets->size(); k++)
                 words = std::max(words, (size_t)(*sets)[k].nshots * fwi::kResSlots * nz * (*sets)[k].pitch);
-        };
-        need(run.fwd);
-        need(run.adj);
         const size_t wmax = (size_t)fwi::kResSlots * fwi::kResMaxCtas;
         if (words > res_words) {
             if (res_x) cudaFree(res_x);
@@ -1722,9 +1817,9 @@ template <typename T> struct Ctx : CtxBase {
             // small shots on chip: one cluster per shot, every step in one launch (prop_cluster.cuh);
             // shots over the whole GPU: one launch per set of shots (prop_resident.cuh)
             ResidentRun resident;
-            const bool on_resident = resident_path(bs, nxm, want_grad, resident);
+            const ResidentBatch in_flight(resident_queue(cfg.device), res_sharing);
+            const bool on_resident = resident_path(bs, nxm, want_grad, in_flight.sharing, resident);
             const bool on_cluster = !on_resident && cluster_path(nxm);
-            ResidentTurn turn(on_resident ? &resident_mutex(cfg.device) : nullptr, st);
             if (!resident.fwd) {
                 for (auto &p : lvl) TRY(cudaMemsetAsync(p, 0, lb, st));
                 for (int k = 0; k < 4; k++) TRY(cudaMemsetAsync(cp[k], 0, lb, st));
@@ -1793,11 +1888,14 @@ template <typename T> struct Ctx : CtxBase {
                     launches++;
                 }
             }
-            if (resident.fwd &&
-                (rc = resident_forward(bf, *resident.fwd, nxm, ntb, 0, ntb,
-                                       !want_grad ? ntb : ckpt ? first_direct * ck_every : 0,
-                                       ckpt ? ck_every : nt_max, -1, ckpt ? first_direct : 0)))
-                return rc;
+            if (resident.fwd) {
+                ResidentTurn turn(resident_queue(cfg.device), st, ev_res[0], resident.ctas(false), n_sm);
+                TRY(turn.err);
+                if ((rc = resident_forward(bf, *resident.fwd, nxm, ntb, 0, ntb,
+                                           !want_grad ? ntb : ckpt ? first_direct * ck_every : 0,
+                                           ckpt ? ck_every : nt_max, -1, ckpt ? first_direct : 0)))
+                    return rc;
+            }
             rc = on_cluster || resident.fwd ? FWI_OK : run_section(section_key(0), 1u, nsamp, spts, [&]() -> int {
                 int cur = 0;
                 for (int g = 0; g < ntb; g++) {
@@ -1856,6 +1954,8 @@ template <typename T> struct Ctx : CtxBase {
             } else if (want_grad && resident.adj) {
                 NvtxRange adj_range("fwi adjoint steps + imaging");
                 for (auto &p : gs) TRY(cudaMemsetAsync(p, 0, lb, st));
+                ResidentTurn turn(resident_queue(cfg.device), st, ev_res[1], resident.ctas(true), n_sm);
+                TRY(turn.err);
                 if (!ckpt) {
                     if ((rc = resident_adjoint(b, *resident.adj, ntb, 0, ntb, 0))) return rc;
                 } else {
