@@ -2491,19 +2491,24 @@ template <typename T> struct Ctx : CtxBase {
         return FWI_OK;
     }
 
-    // fwi_check_bounded_wait: the wait gives up, the status word says so, the
-    // context stays usable (the status word is cleared by every later call).
+    // fwi_check_bounded_wait: each kind of wait (mbarrier, exchanged words) gives up, the status word says
+    // so, the context stays usable (the status word is cleared by every later call).
     int check_bounded_wait(long polls) override
     {
         if (polls < 1 || polls > fwi::kWaitLimit) return FWI_ERR_ARG;
         TRY(cudaMemsetAsync(status, 0, sizeof(unsigned), st));
         k_check_bounded_wait<<<1, 128, 0, st>>>(status, polls);
         TRY_LAUNCH();
-        unsigned stat = 0;
+        unsigned stat = 0, stat2 = 0;
+        int waits[2] = {0, 0};
         TRY(cudaMemcpyAsync(&stat, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        TRY(cudaMemsetAsync(status, 0, sizeof(unsigned), st));
+        TRY(fwi::launch_resident_wait_check(status, polls, (int *)misfit, st));
+        TRY(cudaMemcpyAsync(&stat2, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        TRY(cudaMemcpyAsync(waits, misfit, sizeof(waits), cudaMemcpyDeviceToHost, st));
         TRY(cudaStreamSynchronize(st));
         TRY(cudaMemsetAsync(status, 0, sizeof(unsigned), st));
-        return (stat & fwi::kStatusTimeout) ? FWI_ERR_CUDA : FWI_OK;
+        return (stat & stat2 & fwi::kStatusTimeout) && waits[0] <= polls && waits[1] == 0 ? FWI_ERR_CUDA : FWI_OK;
     }
 
     // Records choice t for the batch shapes the shots form.

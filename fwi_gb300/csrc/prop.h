@@ -227,6 +227,7 @@ struct ResidentSet;
 struct ResFwdArgs;
 struct ResAdjArgs;
 size_t resident_smem_limit();
+cudaError_t launch_resident_wait_check(unsigned *status, long polls, int *waits, cudaStream_t st);
 cudaError_t launch_resident_forward(const Batch<float> &b, const ResidentSet &set, const ResFwdArgs &a, cudaStream_t st);
 cudaError_t launch_resident_adjoint(const Batch<float> &b, const ResidentSet &set, const ResAdjArgs &a, cudaStream_t st);
 cudaError_t launch_resident_ref_adjoint(const Batch<float> &b, const ResidentSet &set, const ResAdjArgs &a,

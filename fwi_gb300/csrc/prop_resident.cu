@@ -29,6 +29,30 @@ ResKernel<ResFwdArgs> fwd_kernel(int store_type, int pitch)
 
 bool resident_allow_ref(int smem);  // prop_resident_ref.cu
 
+// fwi_check_bounded_wait, the resident kernels' wait: a pair of words that nothing writes is polled, given up
+// after `polls`, and the status word says so; the waits after it end at their first poll.
+__device__ __align__(16) uint64_t g_unwritten[2];
+__global__ void k_check_resident_wait(unsigned *status, long polls, int *waits)
+{
+    __shared__ int dead;
+    if (threadIdx.x == 0) dead = 0;
+    __syncthreads();
+    for (int w = 0; w < 2; w++) {
+        int k = 0;
+        for (ResPair q;; k++) {
+            q.load(g_unwritten);
+            if (q.is(1) || res_give_up(k, &dead, status, polls)) break;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) waits[w] = k;
+    }
+}
+cudaError_t launch_resident_wait_check(unsigned *status, long polls, int *waits, cudaStream_t st)
+{
+    k_check_resident_wait<<<1, 128, 0, st>>>(status, polls, waits);
+    return cudaGetLastError();
+}
+
 // Dynamic shared memory of a CTA on the current device (0: the kernels cannot run there): the
 // device's opt-in limit less their static shared memory; the function attributes are set once.
 size_t resident_smem_limit()

@@ -85,10 +85,10 @@ __device__ __forceinline__ uint64_t res_ld1(const uint64_t *p)
 }
 
 // A wait that gave up: the status word and the CTA's flag (its later waits end at once).
-__device__ __forceinline__ bool res_give_up(int polls, volatile int *dead, unsigned *status)
+__device__ __forceinline__ bool res_give_up(int polls, volatile int *dead, unsigned *status, long limit = kWaitLimit)
 {
     if (*dead) return true;
-    if (polls < (int)kWaitLimit) return false;
+    if (polls < limit) return false;
     *dead = 1;
     atomicOr(status, kStatusTimeout);
     return true;

@@ -319,7 +319,8 @@ int fwi_set_tuning(void *ctx, const fwi_shot *shots, int nshots, const fwi_tunin
  * one block waits, as the tile passes wait for their staged tiles, on a
  * barrier phase that nothing completes, gives up after `polls` polls
  * (1 .. 4194304, the tile passes' own limit) and records the timeout in the
- * context's status word.  Returns FWI_ERR_CUDA when the timeout was seen,
+ * context's status word; then the same on a word that nothing writes, as the
+ * resident passes wait for their neighbours' rows.  Returns FWI_ERR_CUDA when both timeouts were seen,
  * as a gradient call would after a wait that gave up; the context stays
  * usable.  No fault, trap or unbounded wait is involved. */
 int fwi_check_bounded_wait(void *ctx, long polls);

@@ -91,3 +91,20 @@ def test_threads_share_the_device():
     seconds(work)
     one = min(seconds(work[:1]) for _ in range(3))
     assert min(seconds(work) for _ in range(3)) < 3 * one
+
+
+@pytest.mark.parametrize("polls", [1, 64, 4096])
+def test_resident_waits_give_up(polls):
+    """The wait for a neighbour's rows, on a word that nothing writes, ends after its polls, is reported,
+    and leaves a context whose resident calls give what they gave."""
+    import fwi_gb300 as f
+    p = exact_problem(seed=2, nx=140, nz=100, nt=120)
+    ctx = f.Context(nx=140, nz=100, dh=p["dh"], dt=p["dt"], cpml=12, f_cpml=p["f"], nt_max=120, max_shots=1)
+    ctx.set_wavelet(wavelet(p).astype(np.float32))
+    ctx.set_model(*(np.ascontiguousarray(p[k], np.float32) for k in ("vh", "vp", "vn")))
+    sh = f.make_shots([dict(sx=70, sz=6, rz=6, rx0=4, rx1=136, nt=120, x0=0, nxw=0)])
+    obs = np.zeros(120 * 132, np.float32)
+    first = ctx.gradient(sh, obs)
+    assert ctx.check_bounded_wait(polls) == -2  # FWI_ERR_CUDA
+    again = ctx.gradient(sh, obs)
+    assert again[0] == first[0] and all(np.array_equal(a, b) for a, b in zip(again[1:], first[1:]))
