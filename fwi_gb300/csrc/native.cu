@@ -771,6 +771,23 @@ struct ResidentTurn {
     } while (0)
 #define TRY_LAUNCH() TRY(cudaGetLastError())
 
+// The state block of a context (Ctx::init): arrays at its start that a checkpointed resident adjoint
+// keeps from one segment to the next; arrays that resident phases may exchange rows in; and the bytes past
+// its end that they may need beyond.
+constexpr size_t kResidentKept = 8;
+inline size_t resident_idle_arrays(const fwi_config &c, bool ckpt)
+{
+    return ckpt ? 6 + 10 : 14 + (c.store == FWI_STORE_FULL ? 0 : 6);
+}
+inline size_t resident_extra_bytes(const fwi_config &c)
+{
+    if (c.precision != FWI_PREC_FP32) return 0;
+    const int win = c.max_window > 0 ? c.max_window : c.nx;
+    const size_t want = fwi::res_exchange_words(c.max_shots, win, c.nz) * sizeof(uint64_t);
+    const size_t idle = resident_idle_arrays(c, c.store == FWI_STORE_CHECKPOINT) * c.max_shots * c.nz * round_up(win, 32) * sizeof(float);
+    return want > idle ? round_up(want - idle, 256) : 0;
+}
+
 template <typename T> struct Ctx : CtxBase {
     int nx = 0, nz = 0, mpitch = 0, pitch = 0, B = 0, nt_max = 0, nrec_max = 0, n_img = 0;
     long slot = 0, mslot = 0;
@@ -980,7 +997,6 @@ template <typename T> struct Ctx : CtxBase {
         drop_sections();
         for (void *p : allocs) cudaFree(p);
         for (const TileListEntry &e : tile_lists) cudaFree(e.dev);
-        if (res_x) cudaFree(res_x);
         for (cudaEvent_t e : ev_res)
             if (e) {
                 ResidentQueue &rq = resident_queue(cfg.device);
@@ -1062,22 +1078,30 @@ template <typename T> struct Ctx : CtxBase {
         TRY(alloc(&cpa, cfg.cpml + 1));
         TRY(alloc(&cpb, cfg.cpml + 1));
         TRY(alloc(&wavelet, nt_max));
-        for (auto &p : lvl) TRY(alloc(&p, (size_t)B * slot));
-        for (auto &p : cp) TRY(alloc(&p, (size_t)B * slot));
+        // the state in one block, arrays of B slots: first what the resident adjoint keeps between the
+        // segments of checkpoint storage, then what no resident phase uses; the rows that resident phases
+        // exchange go there (or over all of it), and past its end what they need beyond
+        std::vector<T **> state = {&lvl[0], &lvl[2], &lvl[4], &lvl[5], &cp[0], &cp[1], &cp[2], &cp[4],
+                                   &lvl[1], &lvl[3], &cp[3], &cp[5], &cp[6], &cp[7]};
+        if (cfg.store != FWI_STORE_FULL)
+            for (T *&p : rlvl) state.push_back(&p);
+        if (cfg.store == FWI_STORE_CHECKPOINT)
+            for (T *&p : rcp) state.push_back(&p);
+        const size_t array = (size_t)B * slot;
+        T *block = nullptr;
+        TRY(alloc(&block, state.size() * array + resident_extra_bytes(cfg) / sizeof(T)));
+        for (size_t k = 0; k < state.size(); k++) *state[k] = block + k * array;
         for (auto &p : gs) TRY(alloc(&p, (size_t)B * slot));
         if (cfg.store == FWI_STORE_CHECKPOINT) {
             ck_every = checkpoint_interval(cfg);
             n_ck = (nt_max + ck_every - 1) / ck_every;
             n_img = 2 * ck_every;  // two segments' images: one rebuilt while the other is consumed
             TRY(alloc(&ck, (size_t)n_ck * 8 * B * slot));
-            for (auto &p : rlvl) TRY(alloc(&p, (size_t)B * slot));
-            for (auto &p : rcp) TRY(alloc(&p, (size_t)B * slot));
         }
         if (cfg.store == FWI_STORE_BOUNDARY) {
             ring_len = fwi::boundary_ring_len(win, nz, cfg.cpml);
             n_img = 2;  // the images of the last two steps rebuilt
             TRY(alloc(&ring, (size_t)B * nt_max * ring_len));
-            for (auto &p : rlvl) TRY(alloc(&p, (size_t)B * slot));
         }
         if (cfg.store != FWI_STORE_FULL) {
             TRY(cudaStreamCreateWithFlags(&rst, cudaStreamNonBlocking));
@@ -1357,9 +1381,9 @@ template <typename T> struct Ctx : CtxBase {
     static constexpr size_t kResidentPlans = 8;
     std::vector<ResidentPlan> resident_plans;  // least recently used first
     fwi::ResWidths resident_widths;
-    uint64_t *res_x = nullptr, *res_w = nullptr;  // exchanged rows and maxima (zeroed when made)
-    size_t res_words = 0;                         // words of the exchanged rows
-    unsigned res_tag = 1;                         // the next unused step tag
+    uint64_t *res_w = nullptr, *res_x = nullptr;  // the batch's exchanged maxima, then rows, in the state block
+    size_t res_bytes = 0;
+    unsigned res_tag = 0;                         // the next unused step tag (0: nothing exchanged yet)
     int res_sharing = 1;                          // the most batches in flight during the last one (ResidentBatch)
     cudaEvent_t ev_res[2] = {};                   // the ends of a batch's forward and adjoint phases (ResidentQueue)
 
@@ -1429,31 +1453,25 @@ template <typename T> struct Ctx : CtxBase {
         }
         size_t words = 0;
         for (const auto *sets : {run.fwd.get(), run.adj.get()})
-            for (size_t k = 0; sets && k < sets->size(); k++)
-                words = std::max(words, (size_t)(*sets)[k].nshots * fwi::kResSlots * nz * (*sets)[k].pitch);
-        const size_t wmax = (size_t)fwi::kResSlots * fwi::kResMaxCtas;
-        if (words > res_words) {
-            if (res_x) cudaFree(res_x);
-            res_x = nullptr;
-            res_words = 0;
-            if (cudaMalloc(&res_x, (words + wmax) * sizeof(uint64_t)) != cudaSuccess) {
-                cudaGetLastError();  // no room for it: the other paths need none
-                res_x = nullptr;
-                run = ResidentRun();
-                return false;
-            }
-            res_w = res_x + words;
-            res_words = words;
-            res_tag = 0xffffffffu;  // zeroed before its first use (resident_tags)
+            for (size_t k = 0; sets && k < sets->size(); k++) words = std::max(words, (*sets)[k].words(nz));
+        // in the arrays past those of a checkpointed adjoint; zeroed before their first use in the batch,
+        // since other phases' values may look like tags
+        res_bytes = ((size_t)fwi::kResSlots * fwi::kResMaxCtas + words) * sizeof(uint64_t);
+        if (res_bytes > resident_idle_arrays(cfg, ckpt) * (size_t)B * slot * sizeof(T) + resident_extra_bytes(cfg)) {
+            run = ResidentRun();
+            return false;
         }
+        res_w = reinterpret_cast<uint64_t *>(lvl[0] + (ckpt ? kResidentKept * B * slot : 0));
+        res_x = res_w + (size_t)fwi::kResSlots * fwi::kResMaxCtas;
+        res_tag = 0;
         return true;
     }
 
-    // Tags of a launch's `steps` steps, never used before in the exchange buffer: the first of them.
+    // Tags of a launch's `steps` steps, used once a batch: the first of them.
     int resident_tags(int steps, unsigned &tag)
     {
-        if (res_tag > 0xffffffffu - (unsigned)steps - 2u) {
-            TRY(cudaMemsetAsync(res_x, 0, (res_words + (size_t)fwi::kResSlots * fwi::kResMaxCtas) * sizeof(uint64_t), st));
+        if (res_tag == 0 || res_tag > 0xffffffffu - (unsigned)steps - 2u) {
+            TRY(cudaMemsetAsync(res_w, 0, res_bytes, st));
             res_tag = 1;
         }
         tag = res_tag;
@@ -1484,6 +1502,7 @@ template <typename T> struct Ctx : CtxBase {
                 a.ck = ck;
                 a.ck_stride = (long)B * slot;
                 a.x = res_x;
+                a.slots = set.slots;
                 a.w = res_w;
                 a.tag0 = tag - (unsigned)g0;
                 TRY(fwi::launch_resident_forward(b, set, a, st));
@@ -1509,6 +1528,7 @@ template <typename T> struct Ctx : CtxBase {
                 a.j1 = j1;
                 a.img_base = img_base;
                 a.x = res_x;
+                a.slots = set.slots;
                 a.tag0 = tag - (unsigned)j0;
                 TRY(exact ? fwi::launch_resident_adjoint(b, set, a, st) : fwi::launch_resident_ref_adjoint(b, set, a, st));
                 launches++;
@@ -2771,6 +2791,7 @@ size_t fwi_config_bytes(const fwi_config *c)
         b += (size_t)c->max_shots * c->nt_max * 2 * slot * se; // images
     }
     b += (size_t)c->max_shots * c->nt_max * nrec * e * 2;  // records and observed data
+    b += resident_extra_bytes(*c);                         // rows exchanged on chip, beyond the idle state
     return b;
 }
 

@@ -13,10 +13,10 @@
 // The exchange goes through L2, value by value: an edge value is stored as 8 bytes, the float and
 // the step it belongs to, and the reader polls the very values it needs.  Neither a fence nor a
 // flag is needed, and the latency is one store and one load.  The per-shot maximum that scales
-// 16-bit images travels the same way (one 8-byte word per CTA).  Words of step t go to copy t mod
-// kResSlots.  No copy is overwritten unread: a CTA that writes step t + 1 has its neighbours' rows
-// of step t, so they have read theirs of step t - 1, the next ones theirs of step t - 2, and CTAs
-// kResReach apart (the farthest that exchange rows) theirs of step t - kResReach.
+// 16-bit images travels the same way (one 8-byte word per CTA).  Rows of step t go to copy t mod
+// slots, one more than the CTAs between the farthest that exchange rows.  No copy is overwritten
+// unread: a CTA that writes step t + 1 has its neighbours' rows of step t, so they have read theirs of
+// step t - 1, the next ones theirs of step t - 2, and CTAs d apart theirs of step t - d.
 // Every wait is bounded; one that gives up sets the status word, and its CTA waits no more.
 //
 // A thread owns 2 columns x R consecutive rows; the z-window of its rows slides through registers.
@@ -293,24 +293,24 @@ __device__ __forceinline__ void res_side_sync(const ResBand &B)
     asm volatile("bar.sync 1, %0;" ::"r"(B.nside_threads) : "memory");
 }
 
-// Exchanged words of interior row gi, columns col, col + 1, of the step with tag.
+// Exchanged words of interior row gi, columns col, col + 1, in copy `copy` of `slots`.
 template <int PT>
-__device__ __forceinline__ uint64_t *res_words(const ResBand &B, uint64_t *x, unsigned tag, int gi, int col)
+__device__ __forceinline__ uint64_t *res_words(const ResBand &B, uint64_t *x, int slots, int copy, int gi, int col)
 {
-    return x + ((long)(B.xs * kResSlots + (int)(tag & (kResSlots - 1))) * B.nz + 4 + gi) * PT + (col - 4);
+    return x + ((long)(B.xs * slots + copy) * B.nz + 4 + gi) * PT + (col - 4);
 }
+__device__ __forceinline__ int res_next(int copy, int slots) { return copy + 1 == slots ? 0 : copy + 1; }
 
-// The halo rows of step `tag` into f (row r of the band at f + r PT): a thread its column pair's
-// rows seg, seg + nlane, ....  Up to U rows are asked for together and those that have not come
-// again, by every thread for itself (one lane polling for its warp measured slower: C1 3.5 us a
-// forward step against 2.9).
+// The halo rows of step `tag` (`base`: the words of the band's first row at the thread's columns) into f
+// (row r of the band at f + r PT): a thread its column pair's rows seg, seg + nlane, ....  Up to U rows
+// are asked for together and those that have not come again, by every thread for itself (one lane
+// polling for its warp measured slower: C1 3.5 us a forward step against 2.9).
 template <int PT>
-__device__ __forceinline__ void res_halo_in(const ResBand &B, float *f, uint64_t *x, unsigned tag, volatile int *dead,
+__device__ __forceinline__ void res_halo_in(const ResBand &B, float *f, const uint64_t *base, unsigned tag, volatile int *dead,
                                             unsigned *status)
 {
     constexpr int U = 6;
     if (!B.use) return;
-    const uint64_t *const base = res_words<PT>(B, x, tag, B.row0, B.ix);
     for (int h0 = B.seg; h0 < 2 * B.hr; h0 += U * B.nlane) {
         ResPair q[U];
         unsigned late = 0;
@@ -489,6 +489,7 @@ k_resident_fwd(const __grid_constant__ Batch<float> b, const __grid_constant__ R
     float *const amax = b.amax + (long)B.s * (b.nt_max + 1);
     int seg = gs / a.period, gseg = gs - seg * a.period;  // segment of the step, step in it
     int cur = 0;                                          // the current level
+    int copy = (int)((a.tag0 + gs) % a.slots);            // ... and the copy of the exchanged rows
     __syncthreads();
     for (int g = gs; g < a.g1; g++) {
         const unsigned tag = a.tag0 + g;
@@ -555,7 +556,8 @@ k_resident_fwd(const __grid_constant__ Batch<float> b, const __grid_constant__ R
                 if (B.self == B.k0) b.scale[(long)B.s * b.nt_max + g] = sc;
             }
         }
-        if (g > gs) res_halo_in<PT>(B, F, a.x, tag, &dead, b.status);
+        if (g > gs) res_halo_in<PT>(B, F, res_words<PT>(B, a.x, a.slots, copy, B.row0, ix), tag, &dead, b.status);
+        copy = res_next(copy, a.slots);
         __syncthreads();
         if (B.bottom) {
             // psi_z of the bottom layer's points of the own rows and 4 either side
@@ -590,7 +592,7 @@ k_resident_fwd(const __grid_constant__ Batch<float> b, const __grid_constant__ R
         if (nr > 0) {
             const float sc = Cd::scaled && img ? s_sc : 1.f;
             SI *const image = (SI *)b.store + ((long)B.s * b.n_img + (img ? gseg + (seg & 1) * a.period : 0)) * 2 * b.slot + i0;
-            uint64_t *const out = res_words<PT>(B, a.x, tag + 1, B.row0 + r0, ix);
+            uint64_t *const out = res_words<PT>(B, a.x, a.slots, copy, B.row0 + r0, ix);
             const float *const fc = F + r0 * PT + ix;
             float *const fn = S.halo[1 - cur] + r0 * PT + ix;
             bool sat = false;
@@ -702,7 +704,7 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
     const long i0 = (long)(B.iz0 + r0) * b.pitch + ix;
     // the next step's u from lambda at row rr, into level `to`, its edge rows to the neighbours: u = g
     // (+ a Z at layer points, Z advanced first, Z' = g + b Z, or not)
-    auto make_u = [&](int rr, int to, const float2 &lp, const float2 &lf, bool advance, unsigned tag) {
+    auto make_u = [&](int rr, int to, const float2 &lp, const float2 &lf, bool advance, unsigned tag, int copy) {
         float *const o = pO + rr * OWN * PT;
         float2 ux = fma(ld2(o + 2 * PT), lp, mul(ld2(o + 4 * PT), lf)), uz = mul(ld2(o + 3 * PT), add(lp, lf));
         const int r = r0 + rr;
@@ -731,10 +733,11 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
             put2(ps + 3 * WB, make_float2(lay0 || zl ? ux.x : 0.f, lay1 || zl ? ux.y : 0.f));
         }
         if (nval < 2) ux.y = uz.y = 0.f;
-        if (B.published(r)) ResPair::put(res_words<PT>(B, a.x, tag, B.row0 + r, ix), uz, tag);
+        if (B.published(r)) ResPair::put(res_words<PT>(B, a.x, a.slots, copy, B.row0 + r, ix), uz, tag);
         put2(o + to * PT, ux);
         put2(S.halo[to] + r * PT + ix, uz);
     };
+    int copy = (int)((a.tag0 + a.j0) % a.slots);  // of the exchanged rows
     float2 LP[R], LF[R], WP[R], WF[R];
     // u of the first step from the loaded lambda and Z (zero at the first iteration); its edge rows out
 #pragma unroll
@@ -758,7 +761,7 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
                 put2(pS + (rr * SD + 1) * WB, ld2(b.cp[2] + i));
             }
             if (B.bottom && B.iz0 + r0 + rr >= B.zb) put2(S.zo + (r0 + rr) * 2 * PT + ix, ld2(b.cp[4] + i));
-            make_u(rr, 0, LP[rr], LF[rr], false, a.tag0 + a.j0);
+            make_u(rr, 0, LP[rr], LF[rr], false, a.tag0 + a.j0, copy);
         }
     }
     if (load && B.bottom && B.use)  // Y_z with 4 rows either side
@@ -833,7 +836,8 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
             for (int rr = 0; rr < nr; rr++)  // -Dx(a Y) within their reach
                 put2(pS + (rr * SD + 4) * WB, scaled(ResWindow(pS + (rr * SD + 2) * WB).d1(), -inv_dh));
         }
-        if (j > a.j0 || load) res_halo_in<PT>(B, UZ, a.x, tag, &dead, b.status);
+        if (j > a.j0 || load) res_halo_in<PT>(B, UZ, res_words<PT>(B, a.x, a.slots, copy, B.row0, ix), tag, &dead, b.status);
+        copy = res_next(copy, a.slots);
         __syncthreads();
         if (REF && B.bottom) {
             // psi_z, then zeta_z and what the bottom layer adds to Dzz u_z, as the forward
@@ -907,7 +911,7 @@ k_resident_adj(const __grid_constant__ Batch<float> b, const __grid_constant__ R
                 if (nval < 2) WP[rr].y = WF[rr].y = 0.f;
                 LP[rr] = add(LP[rr], WP[rr]);
                 LF[rr] = add(LF[rr], WF[rr]);
-                make_u(rr, 1 - cur, LP[rr], LF[rr], true, tag + 1);
+                make_u(rr, 1 - cur, LP[rr], LF[rr], true, tag + 1, copy);
                 if (!img) continue;
                 const SI *const image = images + (long)(g_img - a.img_base) * 2 * b.slot + (long)rr * b.pitch;
                 const float2 gi = keep(mul(kk, Img::value(STAGE ? pI + rr * 2 * PT : image, inv_sc)), nval),

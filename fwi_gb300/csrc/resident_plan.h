@@ -26,8 +26,10 @@ constexpr int kResMaxCtas = 160;  // CTAs of a launch (one per SM)
 constexpr int kResMinRows = 1;
 inline int res_min_rows(int nshots) { return nshots == 1 ? kResMinRows : 2; }
 constexpr int kResReach = (2 * kRad + kResMinRows - 1) / kResMinRows;  // a halo comes from so many CTAs either side at most
-constexpr int kResSlots = 16;     // copies of the exchanged rows (step modulo kResSlots): more than kResReach
-static_assert(kResSlots > kResReach && (kResSlots & (kResSlots - 1)) == 0, "copies of the exchanged rows");
+constexpr int kResSlots = 16;     // copies of the exchanged maxima (step modulo kResSlots)
+static_assert(kResSlots > kResReach && (kResSlots & (kResSlots - 1)) == 0, "copies of the exchanged maxima");
+// Copies of the exchanged rows a launch needs at most (ResidentSet::slots: its farthest exchange and one).
+inline int res_most_slots(int nshots) { return (2 * kRad + res_min_rows(nshots) - 1) / res_min_rows(nshots) + 1; }
 constexpr int kResSide = 96;      // floats of a side array's row
 constexpr int kResMaxCpml = 32;   // the widest layer whose side columns fit one
 constexpr int kResFwdOwn = 5, kResAdjOwn = 8;    // own-row arrays
@@ -68,8 +70,21 @@ struct ResidentGrid {
 struct ResidentSet {
     ResidentGrid grid;
     int pitch, threads, nshots;
+    int slots;  // copies of the exchanged rows (step modulo slots)
     size_t smem;
+    // words of the exchanged rows: [shot][slots][nz][pitch]
+    size_t words(int nz) const { return (size_t)nshots * slots * nz * pitch; }
 };
+
+// Words a context's batches exchange at most: shots in flight, window and rows of the grid.
+inline size_t res_exchange_words(int max_shots, int window, int nz)
+{
+    int pt = 0;
+    for (int p : kResPitches)
+        if (!pt && ((window + 3) / 4 * 4 <= p || p == 640)) pt = p;
+    const size_t row = (size_t)nz * pt, one = res_most_slots(1) * row, all = (size_t)max_shots * res_most_slots(2) * row;
+    return (max_shots > 1 && all > one ? all : one) + (size_t)kResSlots * kResMaxCtas;
+}
 
 // Whose roundings of the CPML terms a forward launch follows: the cluster path's, those of the layer tiles
 // that advance psi themselves, those of the layer tiles after the strip pass.
@@ -86,7 +101,8 @@ struct ResFwdArgs {
     int plain_images;  // images of the plain stencils (reference mode)
     float *ck;       // [checkpoint][8][ck_stride]
     long ck_stride;
-    uint64_t *x;     // exchanged rows: [xs][kResSlots][nz][shared row pitch] words
+    uint64_t *x;     // exchanged rows: [xs][slots][nz][shared row pitch] words
+    int slots;
     uint64_t *w;     // exchanged maxima: [kResSlots][kResMaxCtas] words
     unsigned tag0;   // a word of step g carries tag0 + g
 };
@@ -95,6 +111,7 @@ struct ResFwdArgs {
 struct ResAdjArgs {
     int ntb, j0, j1, img_base;
     uint64_t *x;
+    int slots;
     unsigned tag0;
 };
 
@@ -360,6 +377,14 @@ inline bool resident_plan(const std::vector<int> &nx, int nz, int cpml, size_t s
             }
         }
         g.n = c;
+        // the farthest CTAs that exchange rows
+        for (int a = 0; a < c; a++)
+            for (int d = 1; d <= kResReach && a + d < g.first[a] + g.count[a]; d++) {
+                const int e = g.row0[a] + g.nrow[a], low = g.row0[a + d];
+                if (e + res_halo(g.row0[a], e, nz, cpml) > low || low - res_halo(low, low + g.nrow[a + d], nz, cpml) < e)
+                    set.slots = std::max(set.slots, d);
+            }
+        set.slots++;
         if (set.smem > smem_limit) {  // a grid lower than the bottom layer: not a window the library takes
             out.clear();
             return false;
