@@ -48,7 +48,13 @@ inline void note(cudaError_t e)
 }
 inline void note_launch() { note(cudaGetLastError()); }
 
-inline dim3 tile_grid(int nx, int nz) { return dim3((nx + TX - 1) / TX, (nz + TZ - 1) / TZ); }
+// Tile rows along y, past a grid's 65535 along z too (grids of more than 524280 rows).
+inline dim3 tile_grid(int nx, int nz)
+{
+    const unsigned rows = (nz + TZ - 1) / TZ, y = rows < 65535u ? rows : 65535u;
+    return dim3((nx + TX - 1) / TX, y, (rows + y - 1) / y);
+}
+__device__ __forceinline__ int tile_z0() { return (int)(blockIdx.z * gridDim.y + blockIdx.y) * TZ; }
 
 // The reference's 8th-order stencils (src/parallelcalls.cu:57, 127).  v(k) is the
 // FP32 value k points from the centre along the stencil's axis.  Differences and
@@ -206,7 +212,7 @@ __global__ void k_second_p(const float *__restrict__ P, const float *__restrict_
 {
     __shared__ float sP[TZ][XW];
     __shared__ float sF[ZH][TX];
-    const int x0 = blockIdx.x * TX, z0 = blockIdx.y * TZ;
+    const int x0 = blockIdx.x * TX, z0 = tile_z0();
     fwi::load_xhalo<float, TX, TZ>(sP, P, x0, z0, nx, nz, nx);
     fwi::load_zhalo<float, TX, TZ>(sF, F, x0, z0, nx, nz, nx);
     __syncthreads();
@@ -288,7 +294,7 @@ k_fwd_main(float *p2, float *r2, float *PF, const float *__restrict__ P_pre,
 {
     __shared__ float sP[TZ][XW];
     __shared__ float sF[ZH][TX];
-    const int x0 = blockIdx.x * TX, z0 = blockIdx.y * TZ;
+    const int x0 = blockIdx.x * TX, z0 = tile_z0();
     fwi::load_xhalo<float, TX, TZ>(sP, P_pre, x0, z0, nx, nz, nx);
     fwi::load_zhalo<float, TX, TZ>(sF, F_pre, x0, z0, nx, nz, nx);
     __syncthreads();
@@ -393,7 +399,7 @@ __global__ void __launch_bounds__(TX * TZ) k_adj_main(AdjArgs a)
     __shared__ float s4[ZH][TX];  // aux4 = v_po lambdaF (z-halo)
     __shared__ float sT[ZH][TX];  // snapshot F (z-halo)
     const int nx = a.nx, nz = a.nz;
-    const int x0 = blockIdx.x * TX, z0 = blockIdx.y * TZ;
+    const int x0 = blockIdx.x * TX, z0 = tile_z0();
     stage_x(s1, x0, z0, nx, nz, [&](long i) { return a.v_hor[i] * a.P_pre[i]; });
     stage_x(s3, x0, z0, nx, nz, [&](long i) { return a.v_nmo[i] * a.F_pre[i]; });
     fwi::load_xhalo<float, TX, TZ>(sS, a.P_snap, x0, z0, nx, nz, nx);

@@ -153,10 +153,10 @@ k_fwd_main(Batch<T> b, int g, int ntb, int cur, int img_slot)
 {
     const bool STORE = img_slot >= 0;
     using Cd = Codec<T, ST>;
-    const int s = blockIdx.z;
+    const int plane = blockIdx.z < b.B ? 0 : blockIdx.z / b.B, s = blockIdx.z - plane * b.B;
     const DevShot sh = b.shots[s];
     const int it = g - (ntb - sh.nt);
-    const int x0 = blockIdx.x * PTX, z0 = blockIdx.y * PTZ;
+    const int x0 = blockIdx.x * PTX, z0 = (plane * gridDim.y + blockIdx.y) * PTZ;
     if (it < 0 || x0 >= sh.nx) return;
     const int nx = sh.nx, nz = b.nz, pitch = b.pitch, cpml = b.cpml;
     const long so = (long)s * b.slot;
@@ -368,9 +368,9 @@ __global__ void __launch_bounds__(PTX * PTZ)
 k_adj_main(Batch<T> b, int j, int ntb, int cur, int zsel, int img_base)
 {
     using Cd = Codec<T, ST>;
-    const int s = blockIdx.z;
+    const int plane = blockIdx.z < b.B ? 0 : blockIdx.z / b.B, s = blockIdx.z - plane * b.B;
     const DevShot sh = b.shots[s];
-    const int x0 = blockIdx.x * PTX, z0 = blockIdx.y * PTZ;
+    const int x0 = blockIdx.x * PTX, z0 = (plane * gridDim.y + blockIdx.y) * PTZ;
     if (j >= sh.nt || x0 >= sh.nx) return;
     const int nx = sh.nx, nz = b.nz, pitch = b.pitch, cpml = b.cpml;
     const long so = (long)s * b.slot;
@@ -507,10 +507,12 @@ k_adj_main(Batch<T> b, int j, int ntb, int cur, int zsel, int img_base)
 
 // ---------------------------------------------------------------- launchers
 
+// Tile rows along y, past a grid's 65535 (524280 rows) in further planes of shots along z.
 template <typename T>
 inline dim3 main_grid(const Batch<T> &b, int nx_max)
 {
-    return dim3((nx_max + PTX - 1) / PTX, (b.nz + PTZ - 1) / PTZ, b.B);
+    const unsigned rows = (b.nz + PTZ - 1) / PTZ, y = rows < 65535u ? rows : 65535u;
+    return dim3((nx_max + PTX - 1) / PTX, y, b.B * ((rows + y - 1) / y));
 }
 
 template <typename T>
