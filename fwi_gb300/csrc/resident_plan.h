@@ -76,9 +76,11 @@ struct ResidentSet {
     size_t words(int nz) const { return (size_t)nshots * slots * nz * pitch; }
 };
 
-// Words a context's batches exchange at most: shots in flight, window and rows of the grid.
+// Words a context's batches exchange at most: shots in flight, window and rows of the grid.  (0: more
+// rows than the CTAs hold at the narrowest pitch in 227 KB each, forward rows of own and haloed arrays.)
 inline size_t res_exchange_words(int max_shots, int window, int nz)
 {
+    if (nz - 8 > kResMaxCtas * (int)(232448 / ((kResFwdOwn + 2) * sizeof(float) * kResPitches[0]))) return 0;
     int pt = 0;
     for (int p : kResPitches)
         if (!pt && ((window + 3) / 4 * 4 <= p || p == 640)) pt = p;
