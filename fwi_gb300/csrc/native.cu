@@ -1202,13 +1202,11 @@ template <typename T> struct Ctx : CtxBase {
     // runs their MIXED kernels; the layer passes then take one shot per
     // block).  A block pays for its start (the list of shots, the adjoint's model
     // tiles and gradient sums) once a group; blocks too few or too long leave the last
-    // wave empty.  Forward: 9 blocks an SM (4 resident), adjoint 4 (3 resident).  Adjoint
-    // microseconds a step with 9 -> 4 blocks an SM (with the recompute of checkpoint storage, the
-    // rebuild of boundary storage): 32 of 609 x 309 98.8 -> 96.0, 7 of 700 x 250 33.7 -> 28.5, 3 of
-    // 900 x 600 44.8 -> 35.1, 5 of 800 x 300 (boundary) 37.1 -> 29.2, 24 of 700 x 300 (boundary) 95.3 ->
-    // 93.6 (2 blocks: 107).  Forward with 9 / 7 / 12 blocks: 32 of 609 x 309 48.4 / 50.9 / 49.5, 40 of
-    // 420 x 200 30.8 / 32.8 / 31.6, 24 of 700 x 300 41.7 / 42.2 / 44.0.
-    int shots_per_group(const std::vector<DevShot> &bs, int nxm, bool adjoint) const
+    // wave empty: 9 blocks an SM (4 forward, 3 adjoint ones resident), 6 in an adjoint whose layer tiles
+    // advance the memory variables.  Against 9 in 419 drawn batches, layer tiles as below: 6 gain 1.3 %
+    // (reference mode) to 7 % and lose nowhere more than 1 %, 4 lose up to 9 %; without the
+    // memory variables in the tiles or with several windows 6 lose up to 3 %.
+    int shots_per_group(const std::vector<DevShot> &bs, int nxm, long blocks_per_sm) const
     {
         if (!use_tma) return 1;
         if (const char *e = getenv("FWI_SHOTS_PER_GROUP")) {  // tuning override
@@ -1216,7 +1214,7 @@ template <typename T> struct Ctx : CtxBase {
             if (v >= 1) return std::min(v, 64);
         }
         const long tiles = (long)((nxm - 5) / 32 + 1) * ((nz - 5) / 32 + 1);  // tiles holding interior points
-        const long blocks = (adjoint ? 4L : 9L) * n_sm;
+        const long blocks = blocks_per_sm * n_sm;
         const long nb = (long)bs.size();
         const long groups = std::max(1L, std::min(nb, (blocks + tiles / 2) / tiles));
         const long sg = (nb + groups - 1) / groups;
@@ -1225,24 +1223,39 @@ template <typename T> struct Ctx : CtxBase {
 
     // Shots per group of the layer tiles (with identical windows).  They run on
     // the side stream beside the interior tiles, in blocks that take half an SM's
-    // registers (the adjoint's also half its shared memory): forward about 7/3 blocks an SM, adjoint
-    // 3/4 (its blocks start dear, and an SM with two of them has no room for interior tiles).
-    // Microseconds a forward / adjoint step, 3/2 blocks an SM for both -> this: 32 of 609 x 309
-    // 50.7 / 101.6 -> 48.4 / 98.7 (adjoint with 1/2: 100.0, 1: 100.9), 16 forward 25.2 -> 24.0, 4 of
-    // 2009 x 809 adjoint 112.3 -> 108.4, 4 of 1009 x 409 (full storage) 33.6 -> 29.1, 40 of 420 x 200
-    // 32.8 / 69.4 -> 30.8 / 68.1 (1/2: 72.1).
-    int layer_shots_per_group(int nb, int nxm, int xbase, int zbase, bool adjoint) const
+    // registers (the adjoint's also half its shared memory, and their start is dear).  Blocks an SM, by
+    // what the drawn batches lose and gain against 3/2:
+    //  - forward: 2, as many as are resident (up to 8 %, 1 % lost in one; 7/3 lose up to 7 %); 3/2 where
+    //    the strip pass advances the memory variables.
+    //  - adjoint: 1, or 3/4 where the interior tiles are three times as many (an SM with two layer
+    //    blocks has no room for interior tiles); batches of so few layer tiles that 3/2 an SM take one
+    //    shot each do so (4 to 20 %, 1 % lost in one).  3/4 for all: single batches lose 20 %.
+    //  - reference adjoint and strip pass: 3/2 (3/4 lose up to 32 %).
+    // Forward and reference adjoint: one shot where the interior tiles take one at 9 blocks an SM.
+    int layer_shots_per_group(const std::vector<DevShot> &bs, int nxm, const fwi::TileGrid &tg, bool adjoint) const
     {
         if (const char *e = getenv("FWI_LAYER_SHOTS_PER_GROUP")) {  // tuning override
             const int v = atoi(e);
             if (v >= 1) return std::min(v, 64);
         }
-        long tiles = 0;
-        for (int z0 = zbase; z0 < nz; z0 += fwi::kTileEdge)
-            for (int x0 = xbase; x0 < nxm; x0 += fwi::kTileEdge)
-                tiles += fwi::tile_role(x0, z0, nxm, nz, cfg.cpml + fwi::kRad) == 2;
-        const long slots = adjoint ? 3L * n_sm / 4 : 7L * n_sm / 3;
-        const long groups = std::max(1L, std::min((long)nb, (slots + tiles / 2) / std::max(1L, tiles)));
+        const bool exact = cfg.mode == FWI_MODE_EXACT;
+        const long nb = (long)bs.size();
+        long tiles = 0, interior = 0;
+        for (int z0 = tg.zbase; z0 < nz; z0 += fwi::kTileEdge)
+            for (int x0 = tg.xbase; x0 < nxm; x0 += fwi::kTileEdge) {
+                const int role = fwi::tile_role(x0, z0, nxm, nz, cfg.cpml + fwi::kRad);
+                tiles += role == 2;
+                interior += role == 1;
+            }
+        long slots = 3L * n_sm / 2;
+        if (adjoint && exact && tg.inline_strip) {
+            if (tiles * nb <= slots) return 1;
+            slots = interior >= 3 * tiles ? 3L * n_sm / 4 : n_sm;
+        } else {
+            if ((!adjoint || !exact) && shots_per_group(bs, nxm, 9) == 1) return 1;
+            if (!adjoint && tg.inline_strip) slots = 2L * n_sm;
+        }
+        const long groups = std::max(1L, std::min(nb, (slots + tiles / 2) / std::max(1L, tiles)));
         return (int)std::max(1L, std::min((nb + groups - 1) / groups, 64L));
     }
 
@@ -1289,12 +1302,11 @@ template <typename T> struct Ctx : CtxBase {
     Choice default_choice(const std::vector<DevShot> &bs, int nxm, bool adjoint) const
     {
         Choice c;
-        c.sg = shots_per_group(bs, nxm, adjoint);
         fwi::TileGrid tg;
         if (use_tma && uniform_windows(bs)) tg = fwi::tile_grid(nxm, nz, cfg.cpml);
         c.inline_strip = tg.inline_strip ? 1 : 0;
-        c.sg_layer =
-            use_tma && uniform_windows(bs) ? layer_shots_per_group((int)bs.size(), nxm, tg.xbase, tg.zbase, adjoint) : 1;
+        c.sg = shots_per_group(bs, nxm, adjoint && tg.inline_strip ? 6 : 9);
+        c.sg_layer = use_tma && uniform_windows(bs) ? layer_shots_per_group(bs, nxm, tg, adjoint) : 1;
         return c;
     }
 
