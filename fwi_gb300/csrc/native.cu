@@ -1413,19 +1413,42 @@ template <typename T> struct Ctx : CtxBase {
         return sets;
     }
 
+    // Whether a batch whose window fits the cluster path (`at_once` shots side by side) stays there: a C1-sized
+    // or smaller window's step is bound by latency on either path.  So it does where its clusters run through
+    // in hardly more than its longest shot's steps (each takes its own steps as SMs come free) and the windows
+    // are small, a shot of fewer steps counting for fewer points.  One length: to 15000 points
+    // (cluster / resident ms, 160 steps: 4 shots of 88 x 146 1.15 / 1.20, 7 of 186 x 120 1.30 / 1.20).  Several
+    // lengths: to 18000, since a resident shot's SMs idle until it starts (15 of up to 207 x 67
+    // 1.51 / 1.70, 11 of 85 x 238 1.07 / 1.29).
+    bool keeps_clusters(const std::vector<DevShot> &bs, int at_once) const
+    {
+        std::vector<long> busy(std::min(bs.size(), (size_t)at_once), 0);  // steps of the shots side by side
+        double points = 0;
+        for (const DevShot &d : bs) {  // (longest first)
+            *std::min_element(busy.begin(), busy.end()) += d.nt;
+            points = std::max(points, (double)d.nx * nz * d.nt);
+        }
+        const double longest = bs[0].nt;
+        return *std::max_element(busy.begin(), busy.end()) <= 1.15 * longest &&
+               points <= (bs.back().nt < bs[0].nt ? 18000 : 15000) * longest;
+    }
+
     // Which phases of a batch run resident on chip (prop_resident.cuh): FP32, windows that fit, and
-    // where it measured faster (the same shots, milliseconds on the path given -> resident; not with
-    // FWI_CLUSTER=0, the per-step passes):
-    //  - Small windows (to 12000 points) with all their clusters on the device at once keep the
-    //    cluster path: 400 steps of one 72 x 56 shot 1.91 -> 2.21, one 120 x 100 shot 2.36 -> 2.42;
-    //    beyond, 160 x 160 2.78 -> 2.69, 209 x 209 3.47 -> 2.79, 8 of them 7.39 -> 3.79.
-    //  - Forward (and with checkpoints everything): windows to 256 wide; to 400 in batches of up to
-    //    2 M points.  200 steps tiles -> resident: 40 of 209 x 800 17.5 -> 15.2, 8 of 360 x 300
-    //    3.0 -> 2.5, 12 of 400 x 400 (1.9 M points) 4.5 -> 4.3, 16 (2.6 M) 8.3 -> 8.9 (300 steps); one
-    //    500 x 200 1.7 -> 2.3 (300 steps): wide windows leave a CTA few rows and long halos.
-    //  - Adjoint of stored images: windows to 400 wide; to 640 where all shots run at once.  Tiles ->
-    //    resident: 40 of 320 x 300 11.9 -> 8.1 (200 steps), one 609 x 309 3.4 -> 2.0, three (two
-    //    launches) 6.0 -> 6.4 (300 and 400 steps).
+    // where it measured faster than the path it would otherwise take (not with FWI_CLUSTER=0, the per-step
+    // passes).  What counts against the tile passes is how many launches the shots take: each has the
+    // latency of its steps, and wide windows leave a CTA few rows and long halos.
+    //  - A window that fits the cluster path and does not stay there (keeps_clusters): both phases; the
+    //    forward rounds as that path, so that it does not go to the tiles.
+    //  - Forward: to 224 columns; to 400 in 2 launches.  160 steps tiles -> resident, ms: 31 of 150 x 464
+    //    (4 launches) 3.9 -> 3.2, 7 of 389 x 351 (2) 2.3 -> 1.8, 37 of 338 x 123 (3) 2.6 -> 3.4,
+    //    27 of 250 x 822 (14) 7.9 -> 9.5.
+    //  - Checkpointed gradient (both phases, or neither): to 224 columns; to 320 in 3, to 400 in 2
+    //    launches of the forward, reference mode in 8 (its tile adjoint has twice the memory variables).
+    //    120 steps: 12 of 296 x 448 (3) 7.8 -> 5.9, 17 of 310 x 336 (5) 7.6 -> 9.4, 7 of 378 x 553 (3)
+    //    6.5 -> 7.7, 13 of 327 x 484 in reference mode (5) 12.5 -> 11.0.
+    //  - Adjoint of stored images: to 320 columns and in reference mode to 400; to 400 in 4 launches, to
+    //    640 in one.  24 of 282 x 303 (5 launches) 1.5 times as fast, 16 of 346 x 353 (4) 0.82, 19 of
+    //    351 x 447 (7) 0.85; 4 of 632 x 64 (1) 1.6, 7 of 626 x 458 (7) 0.6.
     // The path does not depend on what else is in flight; with `sharing` batches in flight on the device
     // the launches plan for that share of its SMs, or the largest of more that holds them.
     bool resident_path(const std::vector<DevShot> &bs, int nxm, bool want_grad, int sharing, ResidentRun &run)
@@ -1440,19 +1463,20 @@ template <typename T> struct Ctx : CtxBase {
         const bool full = want_grad && cfg.store == FWI_STORE_FULL;
         if (want_grad && !full && !ckpt) return false;
         const int at_once = cluster_path(nxm);
-        if ((long)nxm * nz <= 12000 && at_once && (int)bs.size() <= at_once) return false;
-        long points = 0;
-        std::vector<int> w;
-        for (const DevShot &d : bs) {
-            w.push_back(d.nx);
-            points += (long)d.nx * nz;
-        }
-        const bool fwd = nxm <= 256 || (nxm <= 400 && points <= 2000000L);
-        const size_t lim = fwd || nxm <= 640 ? fwi::resident_smem_limit() : 0;
+        if (at_once && keeps_clusters(bs, at_once)) return false;
+        const size_t lim = nxm <= 640 ? fwi::resident_smem_limit() : 0;
         if (!lim) return false;
-        if (fwd) run.fwd = resident_sets(w, 0, lim, n_sm);
-        if (full ? nxm <= 640 : ckpt && run.fwd) run.adj = resident_sets(w, (int)store_elem(), lim, n_sm);
-        if (run.adj && nxm > 400 && run.adj->size() > 1) run.adj = nullptr;
+        std::vector<int> w;
+        for (const DevShot &d : bs) w.push_back(d.nx);
+        const bool ref = cfg.mode != FWI_MODE_EXACT;
+        if (nxm <= 400) {
+            run.fwd = resident_sets(w, 0, lim, n_sm);
+            const size_t most = !ckpt ? 2 : ref ? 8 : nxm <= 320 ? 3 : 2;
+            if (!at_once && run.fwd && nxm > 224 && run.fwd->size() > most) run.fwd = nullptr;
+            if (at_once && !run.fwd) return false;
+        }
+        if (full || (ckpt && run.fwd)) run.adj = resident_sets(w, (int)store_elem(), lim, n_sm);
+        if (full && run.adj && nxm > 320 && run.adj->size() > (nxm > 400 ? 1u : ref ? run.adj->size() : 4u)) run.adj = nullptr;
         if (ckpt && !run.adj) run.fwd = nullptr;
         if (!run.any()) return false;
         for (int share = sharing; share > 1; share--) {

@@ -12,6 +12,10 @@ torch = pytest.importorskip("torch")
 
 # name: grid, shots, layer, mode, storage, images, windows of several sizes and lengths, the other choice
 CASES = {
+    "forward in three launches": (338, 123, 37, 14, "exact", "forward", "fp16", False, {"FWI_CLUSTER": "0"}),
+    "forward in fourteen launches": (250, 822, 27, 21, "exact", "forward", "fp16", False, {"FWI_CLUSTER": "0"}),
+    "checkpointed in five launches": (310, 336, 17, 15, "exact", "checkpoint", "fp16", False, {"FWI_CLUSTER": "0"}),
+    "small shots of several lengths": (226, 238, 11, 12, "exact", "full", "fp32", True, {"FWI_RESIDENT": "0"}),
     "reference adjoint": (552, 139, 6, 21, "ref", "full", "fp32", False,
                           {"FWI_SHOTS_PER_GROUP": "1", "FWI_LAYER_SHOTS_PER_GROUP": "1"}),
     "layer tiles of tall windows": (201, 757, 30, 20, "exact", "boundary", "fp16", False,
