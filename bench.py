@@ -458,8 +458,7 @@ def native_arm(args, rank, world, dist):
 
 def single_shot_c1(args, fwi_gb300, torch, dev, steps=10, warmup=3):
     """The plain single-shot gradient (C1: 209 x 209, nt 2000, one shot, full image storage) on the
-    on-chip path (key "cluster": one launch takes the shot through every step of a phase, resident over
-    the whole GPU) and, beside it, on the per-step tile passes (FWI_CLUSTER=0); device-resident inputs,
+    on-chip path (one launch takes the shot through every step of a phase, resident over the whole GPU) and, beside it, on the per-step tile passes (FWI_CLUSTER=0); device-resident inputs,
     CUDA events over `steps` gradients after `warmup`."""
     from fwi_gb300 import synth
     w = synth.WORKLOADS["C1"]()
@@ -467,7 +466,7 @@ def single_shot_c1(args, fwi_gb300, torch, dev, steps=10, warmup=3):
     sprec = {"fp32": fwi_gb300.SPREC_NATIVE, "fp16": fwi_gb300.SPREC_FP16, "bf16": fwi_gb300.SPREC_BF16}[args.store]
     out = {"workload": w.name, "storage": "full", "image_store": args.store, "steps": steps}
     obs = None
-    for name, flag in (("cluster", "1"), ("tile_passes", "0")):
+    for name, flag in (("on_chip", "1"), ("tile_passes", "0")):
         os.environ["FWI_CLUSTER"] = flag
         c = fwi_gb300.Context(nx=w.nx, nz=w.nz, dh=w.dh, dt=w.dt, cpml=w.cpml, f_cpml=w.f, nt_max=w.nt,
                               max_shots=1, max_receivers=w.nx, mode=fwi_gb300.MODE_EXACT,
@@ -502,13 +501,13 @@ def single_shot_c1(args, fwi_gb300, torch, dev, steps=10, warmup=3):
                      "gpt_updates_per_s": round(w.physical_point_updates() / (ms / 1e3) / 1e9, 3)}
         del c
     os.environ.pop("FWI_CLUSTER", None)
-    out["cluster_speedup_over_tile_passes"] = round(out["cluster"]["value"] / out["tile_passes"]["value"], 3)
+    out["on_chip_speedup_over_tile_passes"] = round(out["on_chip"]["value"] / out["tile_passes"]["value"], 3)
     # the same shots in a batch, side by side on the GPU
     nb = 8
     base = w.shots[0]
     many = [dict(base, sx=int(8 + (w.nx - 16) * (k + 0.5) / nb)) for k in range(nb)]
     sh8 = fwi_gb300.make_shots(many)
-    for name, flag in (("cluster_batch_of_8", "1"), ("tile_passes_batch_of_8", "0")):
+    for name, flag in (("on_chip_batch_of_8", "1"), ("tile_passes_batch_of_8", "0")):
         os.environ["FWI_CLUSTER"] = flag
         c = fwi_gb300.Context(nx=w.nx, nz=w.nz, dh=w.dh, dt=w.dt, cpml=w.cpml, f_cpml=w.f, nt_max=w.nt,
                               max_shots=nb, max_receivers=w.nx, mode=fwi_gb300.MODE_EXACT,

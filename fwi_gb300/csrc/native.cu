@@ -586,7 +586,7 @@ struct CtxBase {
     int last_cuda = 0;
     int n_sm = 1;        // streaming multiprocessors of the context's device
     int red_blocks = 2;  // blocks of the reduction kernels: 2 per SM
-    int lb_blocks = 3;   // of the L-BFGS passes: 3 per SM (5 pairs, 2009 x 809: 391 us; 2: 432, 4: 412, 8: 546, before values widened as now)
+    int lb_blocks = 3;   // of the L-BFGS passes: 3 per SM (5 pairs on 2009 x 809 with FP64 conversions: 391 us; 2: 432, 4: 412)
     unsigned eg(long n) const { return elt_grid(n, n_sm); }
     float timing[4] = {0, 0, 0, 0};
     long launches = 0;

@@ -1,8 +1,9 @@
 // Small shots resident on chip (FP32, exact adjoint, every step's images
 // kept): one thread-block cluster per shot, sm_103a.
 //
-// A shot whose grid fits the cluster's shared memory (e.g. 209 x 209) gains
-// nothing from the tile passes' per-step launches: one step of one small shot
+// A shot whose grid fits the cluster's shared memory (to about 209 x 209; in the
+// library's dispatch windows of up to some 120 x 120 points, larger ones run
+// resident over the whole GPU) gains nothing from the tile passes' per-step launches: one step of one small shot
 // is a few microseconds of work, less than the launch and dependency latency
 // of the two tile passes.  Here a cluster of up to 16 CTAs (a non-portable
 // cluster size, enabled per kernel) takes one shot through all its time steps

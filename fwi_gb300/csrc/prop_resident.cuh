@@ -38,7 +38,7 @@
 // them, registers over shared memory up to the point where they spill (spills miss the small L1
 // that this much shared memory leaves), 2 columns a thread (4: C1 3.75 us an adjoint step against
 // 3.3, fewer threads a band).  A 2000-step C1 gradient with FP32 images took 16.8 ms on one 16-CTA
-// cluster, takes 11.9; 8 shots with FP16 images 36.2 -> 18.5 (two waves of clusters before); the
+// cluster, takes 11.7; 8 shots with FP16 images 36.2 -> 18.6 (two waves of clusters before); the
 // adjoint of one 609 x 309 shot 34 -> 20 ms for 3000 steps.
 #pragma once
 
