@@ -1,6 +1,6 @@
-"""The built-in routes and group sizes against the other ones on calls that a wrong choice makes a quarter to
-two thirds slower (the FP32 shapes where rules drawn from fewer shapes did so): device time of the call, the
-least of five, within 12 % of the other choice's."""
+"""The built-in routes and group sizes against the other ones on calls that a wrong choice makes an eighth to
+two thirds slower (the FP32 shapes where rules drawn from fewer shapes did so): device time of the call, or of
+its adjoint where that is what the choice changes, the least of five, within 12 % of the other choice's."""
 import numpy as np
 import pytest
 
@@ -27,10 +27,10 @@ CASES = {
 def test_not_slower_than_the_other_choice(name, monkeypatch):
     import fwi_gb300 as fw
     nx, nz, n, cpml, mode, call, images, uneven, other = CASES[name]
-    nt, rng = 160, np.random.default_rng(1)
+    nt, rng = 160, np.random.default_rng([3, nx, nz, n])
     shots = []
     for k in range(n):
-        w = int(rng.integers(nx // 4, 2 * nx // 5)) if uneven else nx
+        w = int(rng.integers(max(2 * cpml + 16, nx // 10), 2 * nx // 5)) if uneven else nx
         x0 = int(rng.integers(0, nx - w + 1))
         t = int(rng.integers(nt // 4, nt + 1)) if uneven and k else nt
         lo, hi = (x0 + cpml, x0 + w - cpml) if mode == "ref" else (x0 + 4, x0 + w - 4)
@@ -45,6 +45,8 @@ def test_not_slower_than_the_other_choice(name, monkeypatch):
     made = fw.make_shots(shots)
     out = [torch.zeros(nz, nx, device="cuda") for _ in range(3)]
 
+    phase = 2 if "FWI_SHOTS_PER_GROUP" in other else 0  # (the adjoint; the call)
+
     def least():
         t = []
         for k in range(8):  # the first two before their graphs are captured
@@ -52,7 +54,7 @@ def test_not_slower_than_the_other_choice(name, monkeypatch):
                 ctx.forward(made, out=obs)
             else:
                 ctx.gradient(made, obs, None, out=out)
-            t.append(float(ctx.last_timing()[:1].item()) if k > 2 else np.inf)
+            t.append(float(ctx.last_timing()[phase]) if k > 2 else np.inf)
         return min(t)
 
     built_in = least()
