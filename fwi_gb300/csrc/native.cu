@@ -1203,9 +1203,10 @@ template <typename T> struct Ctx : CtxBase {
     // block).  A block pays for its start (the list of shots, the adjoint's model
     // tiles and gradient sums) once a group; blocks too few or too long leave the last
     // wave empty: 9 blocks an SM (4 forward, 3 adjoint ones resident), 6 in an adjoint whose layer tiles
-    // advance the memory variables.  Against 9 in 419 drawn batches, layer tiles as below: 6 gain 1.3 %
-    // (reference mode) to 7 % and lose nowhere more than 1 %, 4 lose up to 9 %; without the
-    // memory variables in the tiles or with several windows 6 lose up to 3 %.
+    // advance the memory variables.  Adjoint steps of 419 batches of random shape (90 .. 2000 x 60 .. 900,
+    // 3 to 40 shots, layer tiles as below), 6 against 9: 2 % faster in the mean, up to 21 %, none
+    // more than 1.3 % slower; 4: 3 % in the mean, but up to 12 % slower; where the strip pass advances
+    // them 6 is up to 3 % slower.
     int shots_per_group(const std::vector<DevShot> &bs, int nxm, long blocks_per_sm) const
     {
         if (!use_tma) return 1;
@@ -1223,14 +1224,15 @@ template <typename T> struct Ctx : CtxBase {
 
     // Shots per group of the layer tiles (with identical windows).  They run on
     // the side stream beside the interior tiles, in blocks that take half an SM's
-    // registers (the adjoint's also half its shared memory, and their start is dear).  Blocks an SM, by
-    // what the drawn batches lose and gain against 3/2:
-    //  - forward: 2, as many as are resident (up to 8 %, 1 % lost in one; 7/3 lose up to 7 %); 3/2 where
-    //    the strip pass advances the memory variables.
+    // registers (the adjoint's also half its shared memory, and their start is dear).  Blocks an SM, with the
+    // time of the same batches against 3/2:
+    //  - forward: 2, as many as are resident: 1.1 % faster in the mean, up to 13 %, one 3 % slower (7/3: up
+    //    to 7 % slower); 3/2 where the strip pass advances the memory variables.
     //  - adjoint: 1, or 3/4 where the interior tiles are three times as many (an SM with two layer
     //    blocks has no room for interior tiles); batches of so few layer tiles that 3/2 an SM take one
-    //    shot each do so (4 to 20 %, 1 % lost in one).  3/4 for all: single batches lose 20 %.
-    //  - reference adjoint and strip pass: 3/2 (3/4 lose up to 32 %).
+    //    shot each do so: 5.6 % faster in the mean, up to 1.5 times, none more than 2 % slower (3/4 for
+    //    all: up to 20 % slower).
+    //  - reference adjoint, and after the strip pass: 3/2 (3/4 up to 32 % slower).
     // Forward and reference adjoint: one shot where the interior tiles take one at 9 blocks an SM.
     int layer_shots_per_group(const std::vector<DevShot> &bs, int nxm, const fwi::TileGrid &tg, bool adjoint) const
     {
